@@ -31,6 +31,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstddef>
 #include <cstdint>
@@ -184,6 +185,27 @@ __device__ __forceinline__ int tile_item(const int* tiles, int n_tiles) {
 __device__ __forceinline__ int index_of(float x) { return __float_as_int(x); }
 __device__ __forceinline__ int index_of(double x) {
   return static_cast<int>(__double_as_longlong(x));
+}
+
+// Programmatic dependent launches (a step's chain of launches): a kernel lets the next one's blocks
+// start beside its own as soon as all of its blocks have, and itself waits for the previous one's end
+// before it reads or writes anything that a launch of the step writes; what it reads before (offsets,
+// rows, face records) no launch writes. previous_done returns 0: an index that a read through the
+// non-coherent path goes by takes it as a summand, so that the read cannot be moved before the wait.
+// Without the launch attribute both do nothing.
+__device__ __forceinline__ void dependents_may_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ int previous_done() {
+  int z;
+  asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, 0;" : "=r"(z) : : "memory");
+  return z;
+}
+
+template <class C>
+__device__ __forceinline__ C index_value(int i) {
+  if constexpr (sizeof(C) == 4) return __int_as_float(i);
+  else return __longlong_as_double(static_cast<long long>(i));
 }
 
 // Interior face records start on 32-byte boundaries in FP64 (96 bytes) but not in fp32 (48).
@@ -448,8 +470,9 @@ __global__ void __launch_bounds__(kBlock) k_boundary_states(Dev<P> d) {
 
 // The minimum over a block of positive doubles' bits, then one atomicMin. Every thread of the
 // block calls it.
+constexpr int kMaxWarps = 32;
 __device__ __forceinline__ void block_min_dt(double dt, bool valid, unsigned long long* target) {
-  __shared__ unsigned long long warp_min[kBlock / 32];
+  __shared__ unsigned long long warp_min[kMaxWarps];
   unsigned long long b = valid && dt > 0.0 ? static_cast<unsigned long long>(__double_as_longlong(dt))
                                            : ~0ULL;
 #pragma unroll
@@ -1099,7 +1122,7 @@ template <class P, bool LIMIT, bool DT, int CHUNK>
 __device__ __forceinline__ void gradients_staged_cells(const Dev<P>& d, double cfl, int local) {
   using C = typename P::C;
   if (block_idle(d)) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long bar;
   const int per_block = blockDim.x / 32;
   const int s0 = blockIdx.x * per_block;
@@ -1416,7 +1439,7 @@ __global__ void __launch_bounds__(128, 6) k_gradients_ring(Dev<P> d, double cfl,
   constexpr int kR16 = 4 / kW;                            // pieces of a stencil row
   constexpr int kGS = D + 1, kRS = 2 * D + 1;             // record and row slots
   static_assert(kGRem == 4 || kGRem == 8, "a record's tail is one word");
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  extern __shared__ __align__(128) unsigned char smem_raw[];
   const int nt = blockDim.x, t = threadIdx.x;
   // Regions, each piece interleaved over the block's threads (conflict-free 128-bit accesses):
   // records' whole pieces, records' tails, rows.
@@ -1514,6 +1537,8 @@ __global__ void __launch_bounds__(128, 6) k_gradients_ring(Dev<P> d, double cfl,
   if constexpr (DT) block_min_dt(dt, live, &d.ctl->dt_bits);
 }
 
+#include "cell_blocks.cuh"
+
 // The CFL step alone (first-order schemes), with the block minimum; `dt_out` for the host.
 template <class P>
 __global__ void __launch_bounds__(256) k_spectral(Dev<P> d, double cfl, int local,
@@ -1522,6 +1547,10 @@ __global__ void __launch_bounds__(256) k_spectral(Dev<P> d, double cfl, int loca
   const int c = tile_item(d.cell_tiles, d.n_cell_tiles);
   const bool live = c >= 0 && c < d.n && cell_active(d, c);
   double dt = 0.0;
+  dependents_may_start();
+  const int z = previous_done();
+  d.prim += z;
+  d.prim_b += z;
   if (live) {
     C wc[5];
     load_prim<P>(d.prim, c, wc);
@@ -1664,7 +1693,8 @@ __device__ __forceinline__ void load_cell_in(const Dev<P>& d, int c, int mode, i
 template <class P>
 __device__ __forceinline__ void finish_cell(const Dev<P>& d, int c, const double* res,
                                             double vol, int mode, int stage, double wa, double wb,
-                                            int last, const CellIn& in, bool store_res = true) {
+                                            int last, const CellIn& in, bool store_res = true,
+                                            typename P::C* w_out = nullptr) {
   using C = typename P::C;
   const bool residual_only = mode == kResidual || mode == kFaceParts;
   if (residual_only || (stage == 0 && store_res)) {
@@ -1716,6 +1746,10 @@ __device__ __forceinline__ void finish_cell(const Dev<P>& d, int c, const double
   C w[5], dq[5];
   prim_of_state(d, nu, w, dq);
   store_prim<P>(d.prim_next, c, w, d.ctl);
+  if (w_out != nullptr) {
+#pragma unroll
+    for (int k = 0; k < 5; ++k) w_out[k] = w[k];
+  }
   if (last) mark_invalid(d, c, dq, res);
 }
 
@@ -1956,6 +1990,8 @@ __device__ __forceinline__ void gather_cell(const Dev<P>& d, int c, const typena
   }
 }
 
+#include "face_blocks.cuh"
+
 // The replicas of the fused stage-0 norms summed into the control's words (one block).
 __global__ void k_norm_collect(const unsigned long long* replicas, Control* ctl) {
   for (int i = threadIdx.x; i < 5 * kWords; i += blockDim.x) {
@@ -2132,6 +2168,8 @@ __global__ void k_case_norm_finish(unsigned long long* words, const double* cell
 // prepares its minimum (CFL).
 __global__ void k_begin(Control* ctl, double dt_fixed, unsigned long long* norm_replicas) {
   const int t = threadIdx.x;
+  dependents_may_start();
+  previous_done();
   for (int i = t; i < 5 * kWords; i += blockDim.x) (&ctl->words[0][0])[i] = 0;
   if (norm_replicas != nullptr)
     for (int i = t; i < kNormReplicas * 5 * kWords; i += blockDim.x) norm_replicas[i] = 0;
@@ -2418,7 +2456,8 @@ struct Tuning {
   int grad_chunk = 4;    // stencil entries loaded together by the gradient kernel: 1, 2, 4 (8 staged)
   int grad_block = 128;  // its threads per block
   int face_mode = 1;     // 0: gather-recompute (each cell computes its faces' fluxes); 1: store-gather;
-                         // 2: store-gather with a step's stage-0 norms summed in its gather
+                         // 2: store-gather with a step's stage-0 norms summed in its gather;
+                         // 3: the fluxes of each face_block cells' faces in shared memory
   int face_block = 128;  // threads per block of the face-flux (or gather-recompute) kernel
   int gather_block = 256;  // threads per block of the store-gather sum
   int grad_mode = 1;     // 0: stencil rows loaded by each thread; 1: staged by TMA bulk copies;
@@ -2429,7 +2468,9 @@ struct Tuning {
                          // bounded for grad_minb blocks of 128 per SM (chunk 2: 7 or 6; chunk 4: 5);
                          // 5 (fp32+acc64): each warp's stencil rows streamed by TMA bulk copies
                          // into a ring of grad_depth shared-memory slots, grad_chunk gathers in
-                         // flight (5-word with grad_narrow)
+                         // flight (5-word with grad_narrow);
+                         // 6: five threads a cell, the neighbourhood records of each 32 or 64 cells
+                         // (grad_block, at most 64) in shared memory
   int grad_widen = 0;    // mode 4: products widened by widen_scaled: 0 none, 1 x and y, 2 all
   int grad_narrow = 0;   // mode 4: 1 gathers neighbours as 16 + 4 bytes instead of 32
   int grad_minb = 7;     // mode 4: blocks of 128 threads per SM the registers are bounded for
@@ -2470,16 +2511,16 @@ struct Tuning {
 
 void Tuning::validate() const {
   auto block_ok = [](int b) { return b >= 32 && b <= 256 && b % 32 == 0; };
-  if (grad_mode == 0 && grad_chunk != 1 && grad_chunk != 2 && grad_chunk != 4)
-    fail("E1101: grad_chunk is 1, 2 or 4");
+  if (grad_mode == 0 && grad_chunk != 1 && grad_chunk != 2 && grad_chunk != 4 && grad_chunk != 8)
+    fail("E1101: grad_chunk is 1, 2 or 4 (8: as 4)");
   if (grad_mode == 0 && grad_chunk == 2 && grad_block > 128)
     fail("E1101: the gradient kernel with 2 entries in flight takes <= 128 threads");
   if (grad_mode == 1 && grad_chunk != 2 && grad_chunk != 4 && grad_chunk != 8)
     fail("E1101: grad_chunk of the staged kernel is 2, 4 or 8");
-  if (face_mode < 0 || face_mode > 2) fail("E1101: face_mode is 0, 1 or 2");
+  if (face_mode < 0 || face_mode > 3) fail("E1101: face_mode is 0 to 3");
   if (grad_mode == 3 && grad_chunk != 2 && grad_chunk != 4 && grad_chunk != 8)
     fail("E1101: grad_chunk of the ring kernel is 2, 4 or 8");
-  if (grad_mode < 0 || grad_mode > 5) fail("E1101: grad_mode is 0 to 5");
+  if (grad_mode < 0 || grad_mode > 6) fail("E1101: grad_mode is 0 to 6");
   if (grad_mode == 5) {
     if (grad_block != 128) fail("E1101: the mode-5 gradient kernel takes 128 threads");
     if (grad_chunk != 2 && grad_chunk != 3) fail("E1101: grad_chunk of mode 5 is 2 or 3");
@@ -2676,7 +2717,7 @@ class Impl final : public Stepper {
     }
     // Stencil of owned cells, sliced, each entry {w_x, w_y, w_z, record}: the record of a cell
     // value (its value index) or of boundary face b's state (n + external ghosts + b).
-    const bool has_stencil =
+    const bool has_stencil = has_stencil_ =
         m.stencil != nullptr && m.stencil_offsets != nullptr && m.stencil_lsq_weight != nullptr;
     std::vector<long long> soff(n_ + 1, 0);
     if (has_stencil)
@@ -2795,13 +2836,23 @@ class Impl final : public Stepper {
     wide_ok_mesh_ = d_.wide_ok;
     d_.stall_polls = 0;
     check(cudaMallocHost(reinterpret_cast<void**>(&head_), kControlHead), "cudaMallocHost");
-    if (tuning_.face_mode != 0) ensure_flux_scratch();
+    check(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking), "stream");
+    check(cudaEventCreateWithFlags(&forked_, cudaEventDisableTiming), "event");
+    check(cudaEventCreateWithFlags(&joined_, cudaEventDisableTiming), "event");
+    choose_defaults();
+    ready_plans();
     check(cudaStreamSynchronize(stream), "create");
   }
 
   ~Impl() override {
     drop_graph();
+    release();
+  }
+  void release() {
     if (head_ != nullptr) cudaFreeHost(head_);
+    if (side_ != nullptr) cudaStreamDestroy(side_);
+    if (forked_ != nullptr) cudaEventDestroy(forked_);
+    if (joined_ != nullptr) cudaEventDestroy(joined_);
   }
 
   long long device_bytes() const override {
@@ -2813,6 +2864,9 @@ class Impl final : public Stepper {
       t += static_cast<long long>(b->bytes());
     for (const auto& b : prim_) t += static_cast<long long>(b.bytes());
     t += static_cast<long long>(recon_.bytes());
+    for (const auto& p : grad_plans_)
+      t += static_cast<long long>(p.off.bytes() + p.list.bytes() + p.active.bytes() + p.st.bytes() + p.inc.bytes());
+    for (const auto& p : face_plans_) t += p.bytes();
     return t;
   }
 
@@ -2830,6 +2884,7 @@ class Impl final : public Stepper {
       for (int k = 0; k < 5; ++k)
         bface_host_[static_cast<long long>(b) * kBface + 8 + k] =
             static_cast<C>(data[k * static_cast<long long>(nb_) + b]);
+    walls_ready_ = false;
     check(cudaMemcpyAsync(bface_.ptr(), bface_host_.data(), bface_host_.size() * sizeof(C),
                           cudaMemcpyHostToDevice, stream), "boundary data");
     check(cudaStreamSynchronize(stream), "boundary data");
@@ -2858,6 +2913,7 @@ class Impl final : public Stepper {
     // As the host (physics/src/euler.cpp:903-912): without reconstruction the faces read no
     // gradients or limiter; unlimited, phi is 1 (written by the gradient kernel).
     second_ = on;
+    ready_plans();
     drop_graph();
   }
 
@@ -2884,6 +2940,7 @@ class Impl final : public Stepper {
   // The primitives of the device state u_ into record buffer 0, where every step starts: a new
   // state, so Control::special is cleared first and set again by k_store if this state needs it.
   void store_state() {
+    walls_ready_ = false;
     check(cudaMemsetAsync(&d_.ctl->special, 0, sizeof(unsigned long long), stream), "special");
     launch(k_store<P>, blocks(n_), kBlock, d_, static_cast<const double*>(u_.as<double>()),
            prim_[0].as<C>());
@@ -2949,6 +3006,7 @@ class Impl final : public Stepper {
     check(cudaMemsetAsync(&d_.ctl->step, 0, sizeof(long long), stream), "reset");
     check(cudaMemsetAsync(&d_.ctl->fault, 0, sizeof(unsigned long long), stream), "reset");
     const StepKey key{cfl, dt, local, rk};
+    ready_walls();
     if (graph) {
       if (graph_exec_ == nullptr || !(key == graph_key_)) capture(key);
       for (long long i = 0; i < n; ++i) {
@@ -3017,6 +3075,7 @@ class Impl final : public Stepper {
     }
     timing_ = true;
     const StepKey key{cfl, dt, local, rk};
+    ready_walls();
     try {
       for (long long i = 0; i < n; ++i) enqueue_step(key);
     } catch (...) {
@@ -3040,7 +3099,8 @@ class Impl final : public Stepper {
   void set_tuning(const Tuning& t) override {
     t.validate();
     tuning_ = t;
-    if (t.face_mode != 0) ensure_flux_scratch();  // never inside a graph capture
+    ready_plans();
+    repack_blocks();
     drop_graph();
   }
 
@@ -3049,7 +3109,8 @@ class Impl final : public Stepper {
   // The autotuner: each candidate launch configuration steps the device state `trial_steps` times
   // (after one untimed step) with event timing; the gradient choices are picked by the gradient
   // kernel's time, then the face choices by the time of the face kernels and the norms (which
-  // face mode 2 sums inside its gather). The state is restored after
+  // face mode 2 sums inside its gather); whole steps then decide between these and a new handle's
+  // choices. The state is restored after
   // every trial, so tuning leaves the solution unchanged. Returns the tuned ms per step.
   double autotune(double cfl, double dt, bool local, int rk, int trial_steps) override {
     need_ranks();  // with ranks, every rank tunes together: the trials make the same exchanges
@@ -3080,79 +3141,94 @@ class Impl final : public Stepper {
     if (second_) {
       double best_ms = 1e300;
       Tuning keep = best;
-      for (int mode : {0, 1, 2, 3})
-      for (int chunk : {1, 2, 4, 8})
-        for (int block : {64, 128, 256}) {
-          if (mode == 0 && chunk == 8) continue;
-          if (mode == 0 && chunk == 2 && block > 128) continue;
-          if (mode == 2 && chunk != 1) continue;
-          if ((mode == 1 || mode == 3) && (chunk == 1 || block > 128)) continue;
-          Tuning t = keep;
-          t.grad_mode = mode;
-          t.grad_chunk = chunk;
-          t.grad_block = block;
-          const double ms = measure(t, kGradients);
-          if (ms < best_ms) {
-            best_ms = ms;
-            best = t;
-          }
+      auto trial = [&](int mode, int chunk, int block, int minb) {
+        Tuning t = keep;
+        t.grad_mode = mode;
+        t.grad_chunk = chunk;
+        t.grad_block = block;
+        t.grad_minb = minb;
+        const double ms = measure(t, kGradients);
+        if (ms < best_ms) {
+          best_ms = ms;
+          best = t;
         }
+      };
+      // (the pipelined, ring and widening forms were never the fastest on any measured case: they stay
+      // open to set_tuning and are not tried)
+      for (int block : {64, 128}) {
+        for (int chunk : {1, 2, 4}) trial(0, chunk, block, 7);
+        for (int chunk : {4, 8}) trial(1, chunk, block, 7);
+      }
       if (sizeof(C) == 4 && limiter_)
-        for (int depth : {4, 8})
-          for (int chunk : {2, 3})
-            for (int narrow : {0, 1}) {
-              Tuning t = keep;
-              t.grad_mode = 5;
-              t.grad_block = 128;
-              t.grad_depth = depth;
-              t.grad_chunk = chunk;
-              t.grad_narrow = narrow;
-              const double ms = measure(t, kGradients);
-              if (ms < best_ms) {
-                best_ms = ms;
-                best = t;
-              }
-            }
-      if (sizeof(C) == 4 && limiter_)
-        for (int shape = 0; shape < 3; ++shape)  // (entries in flight, register bound)
-        for (int widen : {0, 1, 2})
-          for (int narrow : {0, 1})
-            {
-              Tuning t = keep;
-              t.grad_mode = 4;
-              t.grad_block = 128;
-              t.grad_widen = widen;
-              t.grad_narrow = narrow;
-              t.grad_chunk = shape == 2 ? 4 : 2;
-              t.grad_minb = shape == 0 ? 7 : (shape == 1 ? 6 : 5);
-              const double ms = measure(t, kGradients);
-              if (ms < best_ms) {
-                best_ms = ms;
-                best = t;
-              }
-            }
+        for (int minb : {7, 6, 5}) trial(4, minb == 5 ? 4 : 2, 128, minb);
+      // the split form, where the mesh is small enough for it to win
+      if (n_ <= 148 * 2048)
+        for (int block : {32, kSplitCells})
+          if (grad_plan(block) != nullptr) trial(6, 2, block, 7);
     }
     {
       double best_ms = 1e300;
       Tuning keep = best;
-      for (int mode : {0, 1, 2})
-        for (int block : {64, 128, 256})
-          for (int gather : {128, 256}) {
-            if (mode == 0 && gather != 256) continue;
-            if (mode == 2 && n_cases_ > 0) continue;  // the same launches as mode 1
-            Tuning t = keep;
-            t.face_mode = mode;
-            t.face_block = block;
-            t.gather_block = gather;
-            const double ms = measure(t, kFaces);
-            if (ms < best_ms) {
-              best_ms = ms;
-              best = t;
-            }
-          }
+      auto trial = [&](int mode, int block, int gather) {
+        Tuning t = keep;
+        t.face_mode = mode;
+        t.face_block = block;
+        t.gather_block = gather;
+        const double ms = measure(t, kFaces);
+        if (ms < best_ms) {
+          best_ms = ms;
+          best = t;
+        }
+      };
+      const bool small = n_ <= 148 * 512;
+      if (small) trial(0, 64, 256);
+      for (int mode : {1, 2})
+        for (int block : {64, 128})
+          for (int gather : {128, 256})
+            if (mode == 1 || n_cases_ == 0) trial(mode, block, gather);  // mode 2 with cases: as mode 1
+      for (int block : {32, 64, 128})
+        for (int threads : {block, 2 * block, 4 * block, 8 * block})
+          if (threads <= 256 && (block == 128 || small) && face_plan(block) != nullptr) trial(3, block, threads);
     }
-    const double total = measure(best, -1);
+    // Whole steps as they run (their graph; the launches of a step overlap, which the sums above do not
+    // see): the choices found against a new handle's.
+    auto step_ms = [&](const Tuning& t) {
+      tuning_ = t;
+      drop_graph();
+      autan_euler_step_result r{};
+      cudaEvent_t e0 = nullptr, e1 = nullptr;
+      check(cudaEventCreate(&e0), "event");
+      check(cudaEventCreate(&e1), "event");
+      step(cfl, dt, local, rk, 1, true, &r);
+      const int n = 4 * trial_steps;
+      float ms = 1e30f;
+      for (int k = 0; k < 2; ++k) {
+        check(cudaEventRecord(e0, stream), "event");
+        step(cfl, dt, local, rk, n, true, &r);
+        check(cudaEventRecord(e1, stream), "event");
+        check(cudaEventSynchronize(e1), "event");
+        float m = 0.0f;
+        check(cudaEventElapsedTime(&m, e0, e1), "event");
+        ms = std::min(ms, m);
+      }
+      cudaEventDestroy(e0);
+      cudaEventDestroy(e1);
+      restore();
+      return static_cast<double>(ms) / n;
+    };
+    tuning_ = Tuning{};
+    choose_defaults();
+    const Tuning usual = tuning_;
+    ready_plans();
+    double total = step_ms(best);
+    const double other = step_ms(usual);
+    if (other < total) {
+      total = other;
+      best = usual;
+    }
     tuning_ = best;
+    ready_plans();
+    repack_blocks();
     drop_graph();
     return total;
   }
@@ -3196,6 +3272,269 @@ class Impl final : public Stepper {
   }
 
   int slices() const { return std::max(1, (n_ + kSlice - 1) / kSlice); }
+
+  // ---- blocks of cells with their neighbourhoods (cell_blocks.cuh)
+
+  struct GradPlan {
+    bool built = false, fits = false;
+    Buffer off, list, st, inc, active;
+    GradShape shape{};
+    int n_active = -1;   // re-packed launches: blocks to launch over (-1: all)
+  };
+
+  // The gradient plan of `nb` cells per block, built on first use (never inside a capture); null
+  // where a block's neighbourhood does not fit: more candidates than the sort's shared memory
+  // holds, places beyond 16 bits or records beyond the launch's shared memory.
+  GradPlan* grad_plan(int nb) {
+    GradPlan& p = grad_plans_[nb / 32];
+    if (p.built) return p.fits ? &p : nullptr;
+    p.built = true;
+    const int nblk = blocks(n_, nb);
+    long long most = 1;
+    for (int s0 = 0; s0 < nblk; ++s0) {
+      long long sum = 0;
+      for (int c = s0 * nb; c < std::min<long long>(n_, (s0 + 1LL) * nb); ++c) sum += st_.len[c] + inc_.len[c];
+      most = std::max(most, sum);
+    }
+    int cap = 1;
+    while (cap < most && cap < (1 << 20)) cap <<= 1;
+    if (cap > kSortCap) return nullptr;
+    Buffer counts(static_cast<size_t>(nblk) * sizeof(int));
+    const size_t sm = 2ULL * cap * sizeof(int);
+    launch_smem(kControl, k_grad_blocks<P, false>, nblk, nb, sm, d_, cap, counts.as<int>(),
+                static_cast<const int*>(nullptr), static_cast<int*>(nullptr), static_cast<C*>(nullptr),
+                static_cast<C*>(nullptr));
+    std::vector<int> n(nblk), off(nblk + 1, 0);
+    check(cudaMemcpyAsync(n.data(), counts.ptr(), counts.bytes(), cudaMemcpyDeviceToHost, stream), "blocks");
+    check(cudaStreamSynchronize(stream), "blocks");
+    long long run = 0;
+    int largest = 0;
+    for (int i = 0; i < nblk; ++i) {
+      off[i] = static_cast<int>(run);
+      run += n[i];
+      largest = std::max(largest, n[i]);
+      if (run >= std::numeric_limits<int>::max()) return nullptr;
+    }
+    off[nblk] = static_cast<int>(run);
+    GradShape shape{0, 0, nb + largest, 0};
+    const int ns = slices(), per = nb / kSlice;
+    for (int a = 0; a < ns; a += per) {
+      const int e = std::min(a + per, ns);
+      shape.st_rows = std::max(shape.st_rows, st_.start[e] - st_.start[a]);
+      shape.inc_rows = std::max(shape.inc_rows, inc_.start[e] - inc_.start[a]);
+    }
+    for (int c = 0; c < n_; ++c) shape.faces = std::max(shape.faces, inc_.len[c]);
+    if (grad_split_bytes<C>(shape, nb) > kBlockSmem) return nullptr;
+    p.off = upload(off, stream);
+    p.list.alloc(std::max<size_t>(1, static_cast<size_t>(run)) * sizeof(int));
+    p.st.alloc(st_e_.bytes());
+    p.inc.alloc(inc_rec_.bytes());
+    launch_smem(kControl, k_grad_blocks<P, true>, nblk, nb, sm, d_, cap, static_cast<int*>(nullptr),
+                static_cast<const int*>(p.off.template as<int>()), p.list.template as<int>(),
+                p.st.template as<C>(), p.inc.template as<C>());
+    check(cudaStreamSynchronize(stream), "blocks");
+    p.shape = shape;
+    p.fits = true;
+    return &p;
+  }
+  struct FacePlan {
+    bool built = false, fits = false;
+    Buffer first, bfirst, rec, face, bface, inc, inc_start, wfirst, walls, active;
+    int faces = 0;          // the most faces of a block
+    long long interior = 0;  // interior faces over all blocks
+    bool walls_ok = false;  // every boundary face's owner is an owned cell
+    int n_active = -1;
+    long long bytes() const {
+      long long t = 0;
+      for (const Buffer* b : {&first, &bfirst, &rec, &face, &bface, &inc, &inc_start, &wfirst, &walls, &active})
+        t += static_cast<long long>(b->bytes());
+      return t;
+    }
+  };
+
+  // The plans that the tuning's launches take (null where it takes none, or the mesh fits none: the
+  // gradients then take the thread-per-cell form, the faces the store-gather one).
+  GradPlan* split_plan() {
+    if (tuning_.grad_mode != 6 || !second_ || !has_stencil_) return nullptr;
+    return grad_plan(std::min(tuning_.grad_block, kSplitCells));
+  }
+  FacePlan* block_faces() { return tuning_.face_mode == 3 ? face_plan(tuning_.face_block) : nullptr; }
+  // Builds what the tuning's launches need (never inside a graph capture).
+  void ready_plans() {
+    split_plan();
+    const bool in_blocks = block_faces() != nullptr;
+    if (tuning_.face_mode != 0 && !in_blocks) ensure_flux_scratch();
+  }
+  static constexpr int kSortCap = 16384;
+  static constexpr size_t kBlockSmem = 200 * 1024;
+
+  static size_t face_block_smem(const FacePlan& p, int nb) {
+    return 5ULL * static_cast<size_t>(std::max(p.faces, nb)) * sizeof(C);
+  }
+
+  // The face plan of `nb` cells per block, built on first use (never inside a capture); null where a
+  // block's faces do not fit (places beyond 15 bits, the sort's or the launch's shared memory).
+  FacePlan* face_plan(int nb) {
+    FacePlan& p = face_plans_[nb / 32];
+    if (p.built) return p.fits ? &p : nullptr;
+    p.built = true;
+    const int nblk = blocks(n_, nb);
+    long long most = 1;
+    for (int b = 0; b < nblk; ++b) {
+      long long sum = 0;
+      for (long long c = static_cast<long long>(b) * nb; c < std::min<long long>(n_, (b + 1LL) * nb); ++c)
+        sum += inc_.len[c];
+      most = std::max(most, sum);
+    }
+    int cap = 1;
+    while (cap < most && cap < (1 << 20)) cap <<= 1;
+    if (cap > kSortCap) return nullptr;
+    Buffer counts(2ULL * nblk * sizeof(int));
+    const size_t sm = 2ULL * cap * sizeof(int);
+    launch_smem(kControl, k_face_blocks<P, false>, nblk, nb, sm, d_, cap, counts.as<int>(),
+                static_cast<const int*>(nullptr), static_cast<const int*>(nullptr),
+                static_cast<typename P::V*>(nullptr), static_cast<int*>(nullptr), static_cast<int*>(nullptr),
+                static_cast<uint2*>(nullptr), static_cast<const int*>(nullptr));
+    std::vector<int> n(2ULL * nblk), first(nblk + 1, 0), bfirst(nblk + 1, 0);
+    check(cudaMemcpyAsync(n.data(), counts.ptr(), counts.bytes(), cudaMemcpyDeviceToHost, stream), "blocks");
+    check(cudaStreamSynchronize(stream), "blocks");
+    long long run = 0, brun = 0;
+    for (int b = 0; b < nblk; ++b) {
+      first[b] = static_cast<int>(run);
+      bfirst[b] = static_cast<int>(brun);
+      run += n[2 * b];
+      brun += n[2 * b + 1];
+      p.faces = std::max(p.faces, n[2 * b] + n[2 * b + 1]);
+      if (run >= std::numeric_limits<int>::max() || brun >= std::numeric_limits<int>::max()) return nullptr;
+    }
+    first[nblk] = static_cast<int>(run);
+    bfirst[nblk] = static_cast<int>(brun);
+    if (p.faces > 32767 || face_block_smem(p, nb) > kBlockSmem) return nullptr;
+    std::vector<int> start(inc_.start.size());
+    long long rows = 0;
+    for (size_t s = 0; s + 1 < inc_.start.size(); ++s) {
+      start[s] = static_cast<int>(rows);
+      rows += ((inc_.start[s + 1] - inc_.start[s]) / kSlice + 3) / 4 * kSlice;
+    }
+    start.back() = static_cast<int>(rows);
+    p.first = upload(first, stream);
+    p.bfirst = upload(bfirst, stream);
+    p.inc_start = upload(start, stream);
+    p.rec.alloc(std::max<size_t>(1, static_cast<size_t>(run)) * kFace * sizeof(C));
+    p.face.alloc(std::max<size_t>(1, static_cast<size_t>(run)) * sizeof(int));
+    p.bface.alloc(std::max<size_t>(1, static_cast<size_t>(brun)) * sizeof(int));
+    p.inc.alloc(std::max<size_t>(1, static_cast<size_t>(rows)) * sizeof(uint2));
+    launch_smem(kControl, k_face_blocks<P, true>, nblk, nb, sm, d_, cap, static_cast<int*>(nullptr),
+                static_cast<const int*>(p.first.template as<int>()),
+                static_cast<const int*>(p.bfirst.template as<int>()), p.rec.template as<typename P::V>(),
+                p.face.template as<int>(), p.bface.template as<int>(), p.inc.template as<uint2>(),
+                static_cast<const int*>(p.inc_start.template as<int>()));
+    // the boundary faces by their owner's block
+    p.walls_ok = true;
+    std::vector<int> wfirst(nblk + 1, 0), walls(static_cast<size_t>(std::max(nb_, 1)), 0);
+    auto owner_of = [&](int b) {
+      const C x = bface_host_[static_cast<long long>(b) * kBface + 13];
+      if constexpr (sizeof(C) == 4) {
+        int i;
+        std::memcpy(&i, &x, 4);
+        return i;
+      } else {
+        long long l;
+        std::memcpy(&l, &x, 8);
+        return static_cast<int>(l);
+      }
+    };
+    for (int b = 0; b < nb_; ++b) {
+      if (owner_of(b) >= n_) p.walls_ok = false;
+      else ++wfirst[owner_of(b) / nb + 1];
+    }
+    for (int b = 0; b < nblk; ++b) wfirst[b + 1] += wfirst[b];
+    std::vector<int> at(wfirst.begin(), wfirst.end() - 1);
+    for (int b = 0; b < nb_; ++b)
+      if (owner_of(b) < n_) walls[at[owner_of(b) / nb]++] = b;
+    p.interior = run;
+    p.wfirst = upload(wfirst, stream);
+    p.walls = upload(walls, stream);
+    check(cudaStreamSynchronize(stream), "blocks");
+    p.fits = true;
+    return &p;
+  }
+
+  // Whether the step's face launches also write the next boundary states.
+  bool carries_walls() {
+    const FacePlan* f = block_faces();
+    return f != nullptr && !ranked() && nb_ > 0 && f->walls_ok;
+  }
+  // Before steps whose face launches carry the boundary states: those of buffer 0, where they start.
+  void ready_walls() {
+    if (!carries_walls() || walls_ready_) return;
+    launch_as(kBoundary, k_boundary_states<P>, blocks(nb_), kBlock, with_rec(0, 0));
+    walls_ready_ = true;
+  }
+
+  // The launch choices of a new handle, by owned cells and precision. Measured step times (us, graph,
+  // one B200; tets HLLC, channels AUSM+-up or Roe):
+  //   gradients, split / a thread per cell (two entries in flight, 64 threads): fp32+acc64 channel
+  //   4 743 cells 47 / 90, 60 100 cells 99 / 114, 134 175 cells 217 / 199, tets 108 000 cells
+  //   122 / 105; fp64 channel 13 730 cells 79 / 99, warped hexahedra 24 000 cells 144 / 124. The split
+  //   form issues 1.8 times the instructions, so it wins while the chip has issue slots to spare.
+  //   That thread-per-cell form / the staged one: 278 289-cell channel 353 / 466, 2 073 600 tets
+  //   1 410 / 1 430.
+  //   Face blocks / store-gather: hexahedra fp64 8 192 cells 38 / 54, fp32+acc64 channels 4 743 cells
+  //   47 / 66, 31 154 cells 68 / 84, 60 100 cells 99 / 109, batched 571 000 cells 665 / 692,
+  //   1 942 000 cells 1 765 / 1 765; tets 2 073 600 cells 1 472 / 1 410 (faces between blocks are
+  //   computed twice); fp64 tets 38 880 cells 87 / 95, 72 000 cells 166 / 152. Cells and threads a
+  //   block: 256 threads to 32 cells at 8 192 cells (38; 128 threads 43), to 64 at 31 154 (68; 32 to
+  //   128: 70), 128 to 64 at 60 100 (99; 128 to 128: 110), 128 to 128 at 134 175 (199; 128 to 64: 207).
+  void choose_defaults() {
+    const bool f32 = sizeof(C) == 4;
+    const long long per_sm = (static_cast<long long>(n_) + 147) / 148;  // cells
+    int nb = 128, threads = 128;
+    if (per_sm <= 64) nb = 32, threads = 256;
+    else if (f32 && per_sm <= 256) nb = 64, threads = 256;
+    else if (!f32 && per_sm <= 128) nb = 32;
+    else if (f32 && per_sm <= 512) nb = 64;
+    const FacePlan* f = per_sm <= (f32 ? 4096 : 384) ? face_plan(nb) : nullptr;
+    // cell orders whose blocks are not compact (lines or layers of cells) share too many faces between
+    // blocks: beyond small meshes, where launches count, no more than 1.4 computations a face
+    if (f != nullptr && per_sm > 512 && f->interior > 1.4 * nif_) f = nullptr;
+    tuning_.face_block = 64;
+    tuning_.gather_block = 128;
+    if (f != nullptr) {
+      tuning_.face_mode = 3;
+      tuning_.face_block = nb;
+      tuning_.gather_block = threads;
+    }
+    if (!second_ || !has_stencil_) return;
+    tuning_.grad_mode = 0;
+    tuning_.grad_chunk = 2;
+    tuning_.grad_block = 64;
+    if (per_sm <= (f32 ? 512 : 128) && grad_plan(32) != nullptr) {
+      tuning_.grad_mode = 6;
+      tuning_.grad_block = 32;
+    }
+  }
+
+  // Re-packed launches of batched cases: the blocks of the tuning's plans that hold a cell of a
+  // case still stepping.
+  void repack_blocks() {
+    auto blocks_of = [&](int nb, Buffer& buf, int& count) {
+      count = -1;
+      if (n_cell_tiles_ < 0 || active_h_.empty()) return;
+      std::vector<uint8_t> mark(static_cast<size_t>(blocks(n_, nb)), 0);
+      for (int k = 0; k < n_cases_; ++k)
+        if (active_h_[k])
+          for (int64_t b = case_offsets_[k] / nb; b <= (case_offsets_[k + 1] - 1) / nb; ++b) mark[b] = 1;
+      std::vector<int> list;
+      for (size_t b = 0; b < mark.size(); ++b)
+        if (mark[b]) list.push_back(static_cast<int>(b));
+      count = static_cast<int>(list.size());
+      buf = upload(list, stream);
+      check(cudaStreamSynchronize(stream), "active blocks");
+    };
+    if (GradPlan* g = split_plan()) blocks_of(std::min(tuning_.grad_block, kSplitCells), g->active, g->n_active);
+    if (FacePlan* f = block_faces()) blocks_of(tuning_.face_block, f->active, f->n_active);
+  }
 
   // Shared memory of the staged gradient kernel at `block` threads: the largest of its blocks'
   // stencil rows and incidence records (twice the incidences when it also stages their normals
@@ -3274,8 +3613,25 @@ class Impl final : public Stepper {
       check(cudaEventCreate(&after), "event");
       check(cudaEventRecord(before, stream), "event");
     }
-    kernel<<<grid, block, smem, stream>>>(args...);
-    const cudaError_t e = cudaGetLastError();
+    cudaError_t e = cudaSuccess;
+    if (chained_ && !timing_ && !ranked() && static_cast<long long>(grid) * block <= 148LL * 2048) {
+      // in a step's chain: the kernel may start beside the previous one (dependents_may_start)
+      cudaLaunchAttribute chain{};
+      chain.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      chain.val.programmaticStreamSerializationAllowed = 1;
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(static_cast<unsigned>(grid));
+      cfg.blockDim = dim3(static_cast<unsigned>(block));
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = stream;
+      cfg.attrs = &chain;
+      cfg.numAttrs = 1;
+      e = cudaLaunchKernelEx(&cfg, kernel, args...);
+      if (e != cudaSuccess) (void)cudaGetLastError();
+    } else {
+      kernel<<<grid, block, smem, stream>>>(args...);
+      e = cudaGetLastError();
+    }
     if (e != cudaSuccess) {
       char what[160];
       std::snprintf(what, sizeof(what), "kernel launch (kind %d, grid %d, block %d, %zu bytes shared)",
@@ -3314,6 +3670,27 @@ class Impl final : public Stepper {
         const int bs = tuning_.face_block;
         launch_as(kFaces, k_faces_cell<P, F, PL, SE>, cell_grid(bs), bs, d, mode, stage, wa, wb,
                   local, last);
+      });
+      return;
+    }
+    if (block_faces() != nullptr) {
+      FacePlan& p = *block_faces();
+      const int bs = tuning_.face_block;
+      const bool some = repacked() && p.n_active >= 0;
+      // first order: only the next step's spectral radius reads boundary states
+      const bool walls = carries_walls() && (second_ || last);
+      FaceBlocks<P> g{p.first.template as<int>(), p.bfirst.template as<int>(),
+                      p.rec.template as<typename P::V>(), p.face.template as<int>(),
+                      p.bface.template as<int>(), p.inc.template as<uint2>(),
+                      p.inc_start.template as<int>(), walls ? p.wfirst.template as<int>() : nullptr,
+                      p.walls.template as<int>(), some ? p.active.template as<int>() : nullptr, bs};
+      const int nblk = some ? std::max(p.n_active, 1) : blocks(n_, bs);
+      dispatch_faces([&](auto flux, auto planar, auto second) {
+        constexpr int F = decltype(flux)::value;
+        constexpr bool PL = decltype(planar)::value, SE = decltype(second)::value;
+        Chain chain(chained_);
+        launch_smem(kFaces, k_faces_block<P, F, PL, SE>, nblk, std::max(bs, tuning_.gather_block),
+                    face_block_smem(p, bs), d, g, mode, stage, wa, wb, local, last);
       });
       return;
     }
@@ -3476,6 +3853,8 @@ class Impl final : public Stepper {
                             bface_warp_case_h_.size() * sizeof(int), cudaMemcpyDeviceToHost, stream),
             "cases");
     n_cell_tiles_ = n_face_tiles_ = n_bface_tiles_ = -1;
+    active_h_.clear();
+    repack_blocks();
     check(cudaStreamSynchronize(stream), "cases");
   }
 
@@ -3486,8 +3865,10 @@ class Impl final : public Stepper {
     bool all = true;
     for (int k = 0; k < n_cases_; ++k) all = all && active[k] != 0;
     drop_graph();
+    active_h_.assign(active, active + n_cases_);
     if (all) {
       n_cell_tiles_ = n_face_tiles_ = n_bface_tiles_ = -1;
+      repack_blocks();
       return;
     }
     std::vector<int> cells, faces, bfaces;
@@ -3510,6 +3891,7 @@ class Impl final : public Stepper {
     put(cell_tiles_, cells, n_cell_tiles_);
     put(face_tiles_, faces, n_face_tiles_);
     put(bface_tiles_, bfaces, n_bface_tiles_);
+    repack_blocks();
   }
 
   // Grids of the step's launches: over the tiles while cases are re-packed, else every item.
@@ -3698,11 +4080,19 @@ class Impl final : public Stepper {
     }
   }
 
+  // Launches inside take part in a step's chain (programmatic dependent launches).
+  struct Chain {
+    bool& on;
+    const bool was;
+    explicit Chain(bool& f) : on(f), was(f) { on = true; }
+    ~Chain() { on = was; }
+  };
+
   // The loops before the faces on record buffer `in`: boundary states, gradients and limiter;
   // with `dt`, the spectral radius and the CFL step of the step too.
-  void enqueue_cells(int in, bool dt, double cfl, bool local) {
+  void enqueue_cells(int in, bool dt, double cfl, bool local, bool walls = true) {
     const Dev<P> d = with_rec(in, in);
-    if (nb_ > 0) launch_as(kBoundary, k_boundary_states<P>, bface_grid(kBlock, nb_), kBlock, d);
+    if (walls && nb_ > 0) launch_as(kBoundary, k_boundary_states<P>, bface_grid(kBlock, nb_), kBlock, d);
     const int g = cell_grid(kBlock);
     const int loc = local ? 1 : 0;
     if (second_) {
@@ -3710,17 +4100,29 @@ class Impl final : public Stepper {
       const int gs = cell_grid(bs);
       auto go = [&](auto lim, auto with_dt) {
         constexpr bool L = decltype(lim)::value, D = decltype(with_dt)::value;
+        if (split_plan() != nullptr) {
+          const GradPlan& g = *split_plan();
+          const int cells = std::min(bs, kSplitCells);
+          const bool some = repacked() && g.n_active >= 0;
+          GradBlocks<P> gb{g.off.template as<int>(), g.list.template as<int>(), g.st.template as<C>(),
+                           g.inc.template as<C>(), some ? g.active.template as<int>() : nullptr};
+          const int nblk = some ? std::max(g.n_active, 1) : blocks(n_, cells);
+          Chain chain(chained_);
+          launch_smem(kGradients, k_gradients_split<P, L, D>, nblk, kSplit * cells,
+                      grad_split_bytes<C>(g.shape, cells), d, gb, g.shape, cfl, loc);
+          return;
+        }
         if (repacked()) {
           launch_as(kGradients, k_gradients_tiles<P, L, D>, cell_grid(128), 128, d, cfl, loc);
           return;
         }
-        if (tuning_.grad_mode == 4 || tuning_.grad_mode == 5) {
+        if (tuning_.grad_mode >= 4) {
           if constexpr (std::is_same_v<P, Fp32Acc64> && L) {
+            if (tuning_.grad_mode == 4) launch_gradients_w<D>(d, cfl, loc);
             if (tuning_.grad_mode == 5) launch_gradients_ring<D>(d, cfl, loc);
-            else launch_gradients_w<D>(d, cfl, loc);
-            return;
+            if (tuning_.grad_mode != 6) return;
           }
-          // fp64 or no limiter: the mode-0 form with two entries in flight
+          // fp64, no limiter, or a mesh that fits no split blocks: the mode-0 form with two entries in flight
           if constexpr (sizeof(C) == 4)
             launch_as(kGradients, k_gradients_occ7<P, L, D>, cell_grid(128), 128, d, cfl, loc);
           else
@@ -3776,6 +4178,7 @@ class Impl final : public Stepper {
         else go(std::false_type{}, std::false_type{});
       }
     } else if (dt) {
+      Chain chain(chained_);
       launch_as(kSpectral, k_spectral<P>, g, kBlock, d, cfl, loc, static_cast<double*>(nullptr));
     }
   }
@@ -3854,6 +4257,8 @@ class Impl final : public Stepper {
     // the stage-0 norms fused into the store-gather sum (not with batched cases, whose per-case
     // norms read the stored residual)
     const bool fused = tuning_.face_mode == 2 && n_cases_ == 0;
+    const bool carried = carries_walls();
+    if (!carried) walls_ready_ = false;
     launch(k_begin, 1, 256, d_.ctl, cfl_dt ? 0.0 : k.dt,
            fused ? norm_words_.as<unsigned long long>() : static_cast<unsigned long long*>(nullptr));
     const int stages = k.rk == 3 ? 3 : 4;
@@ -3865,7 +4270,7 @@ class Impl final : public Stepper {
       const int in = k.rk == 3 ? in3[st] : in4[st];
       const int out = k.rk == 3 ? out3[st] : out4[st];
       if (ranked()) halo(0, prim_[in].as<C>());
-      enqueue_cells(in, st == 0 && cfl_dt, k.cfl, local);
+      enqueue_cells(in, st == 0 && cfl_dt, k.cfl, local, !carried && (second_ || st == 0));
       if (ranked()) {
         if (st == 0 && cfl_dt) reduce_words(&d_.ctl->dt_bits, 1, 1);
         if (second_) halo(1, recon_.as<C>());
@@ -3875,6 +4280,8 @@ class Impl final : public Stepper {
       launch_faces(with_rec(in, out), k.rk == 3 ? kRk3 : kRk4, st, wa, wb, local ? 1 : 0,
                    st == stages - 1 ? 1 : 0, fused && st == 0);
       if (st == 0) {
+        // the norms beside the stages that follow: nothing in them reads or writes what these do
+        Side side(*this, !ranked() && !timing_);
         if (fused) {
           launch_as(kNorms, k_norm_collect, 1, 512,
                     static_cast<const unsigned long long*>(norm_words_.as<unsigned long long>()),
@@ -3902,8 +4309,29 @@ class Impl final : public Stepper {
                     n_cases_, static_cast<const Control*>(d_.ctl), case_hist_.as<double>());
       }
     }
+    if (!ranked() && !timing_) {
+      check(cudaEventRecord(joined_, side_), "join");
+      check(cudaStreamWaitEvent(stream, joined_, 0), "join");
+    }
     if (n_cases_ > 0) launch(k_end_step, 1, 32, d_.ctl);  // after the per-case history
   }
+
+  // With `on`, the launches inside go to the side stream, after what the handle's stream holds so far;
+  // enqueue_step joins it at its end.
+  struct Side {
+    Impl& h;
+    const bool on;
+    cudaStream_t main;
+    Side(Impl& impl, bool use) : h(impl), on(use), main(impl.stream) {
+      if (!on) return;
+      check(cudaEventRecord(h.forked_, main), "fork");
+      check(cudaStreamWaitEvent(h.side_, h.forked_, 0), "fork");
+      h.stream = h.side_;
+    }
+    ~Side() { h.stream = main; }
+    Side(const Side&) = delete;
+    Side& operator=(const Side&) = delete;
+  };
 
   void capture(const StepKey& k) {
     drop_graph();
@@ -3973,8 +4401,16 @@ class Impl final : public Stepper {
   int n_cell_tiles_ = -1, n_face_tiles_ = -1, n_bface_tiles_ = -1;
   std::vector<int64_t> case_offsets_;
   std::vector<int> face_warp_case_h_, bface_warp_case_h_;
+  std::vector<uint8_t> active_h_;  // the active flags of the last set_active
+  bool has_stencil_ = false;
+  GradPlan grad_plans_[5];  // by cells per block / 32
+  FacePlan face_plans_[9];
+  bool walls_ready_ = false;  // buffer 0 holds the boundary states of its primitives
+  bool chained_ = false;  // set around launches of kernels that wait for the previous one themselves
   bool step_tiles_ = false;  // set while enqueue_step records: its launches use the tiles
   Control* head_ = nullptr;  // pinned copy of the control's head
+  cudaStream_t side_ = nullptr;  // a step's norms, beside its later stages
+  cudaEvent_t forked_ = nullptr, joined_ = nullptr;
   struct Timed {
     int kind;
     cudaEvent_t before, after;

@@ -170,7 +170,9 @@ int autan_euler_device_kernel_times(void* handle, double cfl, double dt, int32_t
  * its threads per block, [2] face strategy (0 gather-recompute: each cell recomputes its faces'
  * fluxes; 1 store-gather: each face's flux once into a face scratch, then summed per cell; 2 as 1,
  * with a step's stage-0 residual norms summed inside the gather instead of a pass over a stored
- * residual, without batched cases), [3]
+ * residual, without batched cases; 3: each block of [3] cells computes its cells' faces into shared
+ * memory with [4] threads, at least [3], and sums them there, one launch for fluxes, sums, stage
+ * update and the next boundary states), [3]
  * threads per block of the face kernel, [4] of the store-gather sum, [5] gradient staging (0:
  * each thread loads its stencil rows; 1: each block's rows staged into shared memory by TMA bulk
  * copies, at most 128 threads per block; 2: as 0, software-pipelined: the next entry's gather and
@@ -183,7 +185,11 @@ int autan_euler_device_kernel_times(void* handle, double cfl, double dt, int32_t
  * threads per SM the registers are bounded for: 7 or 6 with [0] = 2, 5 with [0] = 4; 5,
  * fp32+acc64 only: each warp's
  * stencil rows streamed by TMA bulk copies into a ring of [9] (4 or 8) shared-memory slots ahead of
- * the warp, [0] (2 or 3) gathers in flight, [7] as for 4, 128 threads per block).
+ * the warp, [0] (2 or 3) gathers in flight, [7] as for 4, 128 threads per block; 6: five threads per
+ * cell, the rows and neighbour records of each block of [1], at most 64, cells in shared memory). A
+ * new handle takes face mode 3 and gradient staging 6 on small meshes; a mesh whose blocks do not fit
+ * (65 535 or more records or 32 768 faces in one, or its shared memory) takes face mode 1 and staging
+ * 0 in their place.
  * Every choice gives the same bits. No counterpart in the reference beyond its Strategy enum
  * (codegen/include/autan/kernels/strategy.hpp:14-21). */
 int autan_euler_device_set_tuning(void* handle, const int32_t* params, int32_t count, char* err,

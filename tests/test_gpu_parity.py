@@ -271,6 +271,50 @@ def test_gradient_stagings_agree_on_the_channel(precision):
         assert bits_equal(r, norms[(0, 1, 128)]), k
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp32+acc64"])
+@pytest.mark.parametrize("build", [
+    lambda p: cases.vortex_tets(16, 16, 6, steps=3, precision=p),
+    lambda p: cases.vortex_tets(5, 4, 4, steps=3, precision=p),  # 480 cells: part of the last block
+    lambda p: cases.bump_channel(24, 10, 4, steps=3, precision=p, order="rcm"),
+    lambda p: cases.vortex_hex(17, 15, 3, steps=2, precision=p),
+], ids=["tets", "tets-480", "channel", "hex"])  # fmt: skip
+def test_block_forms_are_bit_identical(build, precision):
+    """The split gradients (mode 6, 32 and 64 cells a block) and the face blocks (mode 3, every block
+    of cells with one to eight threads a cell) against the store-gather and thread-per-cell forms:
+    states, norms and steps bit for bit, in graphs and eager, and again after a change of form and of
+    the boundary data between steps (the face blocks carry the boundary states from step to step)."""
+    case = build(precision)
+    data = case.bc_data * 1.001
+    plain = dict(grad_mode=0, grad_chunk=1, grad_block=128, face_mode=1, face_block=128, gather_block=128)
+    split = [dict(grad_mode=6, grad_block=b) for b in (32, 64, 128)]
+    blocks = [dict(face_mode=3, face_block=b, gather_block=t)
+              for b in (32, 64, 128, 256) for t in (32, 128, 256)]
+
+    def march(tuning, graph=True, between=None):
+        with EulerDevice(case.mesh, case.scheme, case.bc_kind, case.bc_data) as dev:
+            dev.set_tuning(**tuning)
+            dev.upload(case.u0)
+            out = []
+            for i in range(2):
+                r = dev.step(cfl=case.cfl, local=case.local, rk=case.rk, n_steps=case.steps, graph=graph)
+                out += [dev.download(), dev.history(case.steps)[0], np.array([r.time_step])]
+                if i == 0:
+                    dev.set_boundary_data(data)
+                    if between:
+                        dev.set_tuning(**between)
+            out.append(dev.residual(case.u0))
+            return out
+
+    want = march(plain)
+    trials = [(dict(plain, **s), True, None) for s in split]
+    trials += [(dict(plain, **b), i % 3 != 0, None) for i, b in enumerate(blocks)]
+    trials += [(dict(plain, **split[0], **blocks[0]), True, plain), (plain, True, dict(split[1], **blocks[4])),
+               (dict(split[0], **blocks[5]), False, None)]
+    for tuning, graph, between in trials:
+        for a, b in zip(march(tuning, graph, between), want):
+            assert bits_equal(a, b), (tuning, graph, between)
+
+
 def test_autotune_leaves_the_solution_unchanged():
     case = cases.vortex_tets(20, 20, 6, steps=3, precision="fp32+acc64")
     a, *_ = run_device(case, case.steps)

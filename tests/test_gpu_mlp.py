@@ -89,6 +89,38 @@ def test_wall_distance_bit_for_bit():
         assert np.array_equal(got[k], np.array(want))
 
 
+@pytest.mark.parametrize("n_tri", [1, 4, 5, 33, 257, 2100])
+def test_wall_distance_through_the_tree(n_tri):
+    """Trees of one to five levels, whole and part leaves: a bumpy wall's triangles (in order and
+    shuffled), thin and degenerate ones among them, a case without triangles and points on, near and
+    far from the wall: the least of every triangle's distance bit for bit."""
+    rng = np.random.default_rng(n_tri)
+    k = np.arange(n_tri)
+    a = np.stack([0.01 * k, 0.05 * np.sin(k), 0.03 * np.cos(3 * k)], axis=1)
+    t = np.concatenate([a, a + rng.normal(scale=0.01, size=(n_tri, 3)),
+                        a + rng.normal(scale=0.01, size=(n_tri, 3))], axis=1)  # fmt: skip
+    t[::7, 6:9] = t[::7, 3:6] + 1e-9 * rng.normal(size=t[::7, 3:6].shape)  # thin
+    t[::31, 3:6] = t[::31, 0:3]  # no area
+    shuffled = t[rng.permutation(n_tri)] + 1000.0
+    near = t[rng.integers(0, n_tri, 12), 0:3].T + rng.normal(scale=1e-3, size=(3, 12))
+    far = rng.normal(scale=30.0, size=(3, 6))
+    pts = np.concatenate([near, far, t[:1, 3:6].T], axis=1)
+    tris, points = [t, np.zeros((0, 9)), shuffled], [pts, pts[:, :2], pts + 1000.0]
+    got = wall_distance(tris, points)
+    assert np.isinf(got[1]).all()
+
+    def distance(p, q):  # a triangle without area can give 0 / 0, which the minimum passes over
+        try:
+            d = O.point_triangle(p, q[0:3], q[3:6], q[6:9])
+        except ZeroDivisionError:
+            return np.inf
+        return np.inf if np.isnan(d) else d
+
+    for c in (0, 2):
+        want = [min(distance(p, q) for q in tris[c]) for p in points[c].T]
+        assert np.array_equal(got[c], np.array(want))
+
+
 @pytest.mark.parametrize("rows", [5000, 40000])
 def test_engines_agree(rows):
     """tcgen05 per layer, fused tcgen05 (tensor memory accumulators) and mma.sync: the same BF16

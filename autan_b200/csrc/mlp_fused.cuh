@@ -241,7 +241,7 @@ __device__ __forceinline__ int job_layer(const Layout& P, int j) {
 template <bool TRAIN>
 __global__ void __launch_bounds__(kThreads, 1)
     k_fused(Layout P, const float* x, const float* y, const int* idx, int rows, int tiles,
-            float* zbuf, unsigned char* atbuf, float* partial, long long count, float* se,
+            float* zbuf, unsigned char* atbuf, float* partial, long long stride, float* se,
             float scale, float* yout, unsigned int* fault) {
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ __align__(8) unsigned long long mma_bar, ld_bar[2], dead_bar;
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int jobs = TRAIN ? 2 * L : L;
   float* const zc = TRAIN ? zbuf + static_cast<long long>(blockIdx.x) * (L - 1) * 128 * 128 : nullptr;
   unsigned char* const atc = TRAIN ? atbuf + static_cast<long long>(blockIdx.x) * P.at_bytes : nullptr;
-  float* const part = TRAIN ? partial + static_cast<long long>(blockIdx.x) * count : nullptr;
+  float* const part = TRAIN ? partial + static_cast<long long>(blockIdx.x) * stride : nullptr;
   // phases: bit b of ld_par is the parity of buffer b's next load; ld_busy bit b: a load issued
   // into buffer b and not yet waited for (thread 0's record, for the fault path)
   uint32_t mma_par = 0, ld_par = 0, ld_busy = 0;
@@ -438,15 +438,14 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
           for (int e = 0; e < 8; ++e) z[e] = acc[8 * j + e] + sbias[c0 + e];
           if (!last) {
-            if constexpr (TRAIN) {
-              // GELU'(Z) for the backward pass (the same erf as the activation's)
-#pragma unroll
-              for (int e = 0; e < 8; ++e)
-                zc[(static_cast<long long>(l) * 128 + c0 + e) * 128 + row] = gelu_grad(z[e]);
-            }
             float a[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) a[e] = gelu(z[e]);
+            for (int e = 0; e < 8; ++e) {
+              float dy;
+              gelu_pair(z[e], &a[e], &dy);
+              // GELU'(Z) for the backward pass
+              if constexpr (TRAIN) zc[(static_cast<long long>(l) * 128 + c0 + e) * 128 + row] = dy;
+            }
             put8(aimg, row, c0, a);
           } else if constexpr (!TRAIN) {
             if (valid)
@@ -509,6 +508,20 @@ __global__ void __launch_bounds__(kThreads, 1)
           for (int j = 0; j < 2; ++j) {
             const int c0 = cb + 8 * j;
             if (16 * half + 8 * j >= cw || c0 >= nw) break;
+            if (direct && P.in[l] == 128) {
+              // this thread's row of W_l, eight columns: one 32-byte store (4-byte ones put each lane of
+              // a warp on a line of its own, 32 wavefronts a word)
+              float* dst = pw + static_cast<long long>(row) * 128 + c0;
+              if (!first) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) wv[8 * j + e] = dst[e] + wv[8 * j + e];
+              }
+              asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "f"(wv[8 * j]),
+                           "f"(wv[8 * j + 1]), "f"(wv[8 * j + 2]), "f"(wv[8 * j + 3]), "f"(wv[8 * j + 4]),
+                           "f"(wv[8 * j + 5]), "f"(wv[8 * j + 6]), "f"(wv[8 * j + 7])
+                           : "memory");
+              continue;
+            }
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
               const int o = direct ? row : c0 + e, i = direct ? c0 + e : row;
@@ -569,15 +582,16 @@ __global__ void __launch_bounds__(kThreads, 1)
 // (as k_adam); with PACK, its BF16 copies into the layer's two operand images (weights only).
 // Nothing is written after a fault of the pass (fault word set; null: no pass).
 template <bool ADAM, bool PACK>
-__global__ void k_fused_update(Layout P, const float* partial, int ctas, long long count,
-                               float* grad, float* params, float* m, float* v, float lr, float c1,
+__global__ void k_fused_update(Layout P, const float* partial, int ctas, long long stride,
+                               long long count, float* grad, float* params, float* m, float* v, float lr, float c1,
                                float c2, const unsigned int* fault) {
   const long long p = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (p >= count) return;
   if (fault != nullptr && *reinterpret_cast<const volatile unsigned int*>(fault) != 0u) return;
   if (partial != nullptr) {
     float s = 0.0f;
-    for (int c = 0; c < ctas; ++c) s += partial[static_cast<long long>(c) * count + p];
+#pragma unroll 16
+    for (int c = 0; c < ctas; ++c) s += partial[static_cast<long long>(c) * stride + p];
     grad[p] = s;
     if constexpr (ADAM) {
       m[p] = 0.9f * m[p] + 0.1f * s;

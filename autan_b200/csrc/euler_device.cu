@@ -49,6 +49,7 @@
 #include "euler_bodies.cuh"
 #include "convergence.hpp"
 #include "exact_sum.cuh"
+#include "host_stage.hpp"
 
 namespace autan_b200 {
 
@@ -2850,6 +2851,7 @@ class Impl final : public Stepper {
   }
   void release() {
     if (head_ != nullptr) cudaFreeHost(head_);
+    if (rows_host_ != nullptr) cudaFreeHost(rows_host_);
     if (side_ != nullptr) cudaStreamDestroy(side_);
     if (forked_ != nullptr) cudaEventDestroy(forked_);
     if (joined_ != nullptr) cudaEventDestroy(joined_);
@@ -2917,24 +2919,64 @@ class Impl final : public Stepper {
     drop_graph();
   }
 
-  // Host state (5 x n_cells, caller-owned; pinned memory makes the copies asynchronous DMA):
-  // one copy per component, of the owned cells.
+  // Host state (5 x n_cells, caller-owned; pinned memory makes the copies asynchronous DMA), the owned
+  // cells of each component: one copy of five rows where the host memory is pinned or the state small,
+  // else (from 8 MB a component) a copy per component through the pinned slots of host_stage.hpp.
+  static constexpr size_t kRowsAtOnce = size_t(1) << 23, kRowsPinned = size_t(1) << 20;
+  bool rows_at_once(const double* host) const {
+    return static_cast<size_t>(n_) * sizeof(double) < kRowsAtOnce || HostStage::pinned(host);
+  }
   void copy_in(const double* host, double* dev) {
     const size_t per = static_cast<size_t>(n_) * sizeof(double);
+    if (rows_at_once(host)) {
+      check(cudaMemcpy2DAsync(dev, per, host, static_cast<size_t>(nc_) * sizeof(double), per, 5,
+                              cudaMemcpyHostToDevice, stream), "upload");
+      return;
+    }
+    if (!in_stage_) in_stage_ = HostStage::of_device(0);
+    ++copies_in_;
     for (int k = 0; k < 5; ++k)
-      check(cudaMemcpyAsync(dev + k * static_cast<long long>(n_), host + k * static_cast<long long>(nc_),
-                            per, cudaMemcpyHostToDevice, stream), "upload");
+      check(in_stage_->to_device(dev + k * static_cast<long long>(n_), host + k * static_cast<long long>(nc_),
+                                 per, stream, copies_in_ > 1), "upload");
   }
-  void copy_out(const double* dev, double* host) {
+  // The images of owned cells in a host array: their owner's values, or zero.
+  void fill_images(double* host, bool zero) const {
+    for (int k = 0; k < 5; ++k)
+      for (int g = n_; g < nc_; ++g) {
+        double* row = host + k * static_cast<long long>(nc_);
+        if (zero) row[g] = 0.0;
+        else if (ghost_owner_[g - n_] >= 0) row[g] = row[ghost_owner_[g - n_]];  // external: left as it is
+      }
+  }
+  void copy_out(const double* dev, double* host, bool zero_images = false) {
     const size_t per = static_cast<size_t>(n_) * sizeof(double);
-    for (int k = 0; k < 5; ++k)
-      check(cudaMemcpyAsync(host + k * static_cast<long long>(nc_), dev + k * static_cast<long long>(n_),
-                            per, cudaMemcpyDeviceToHost, stream), "download");
-    check(cudaStreamSynchronize(stream), "download");
-    for (int k = 0; k < 5; ++k)
-      for (int g = n_; g < nc_; ++g)
-        if (ghost_owner_[g - n_] >= 0)  // an external ghost's entry is left as it is
-          host[k * static_cast<long long>(nc_) + g] = host[k * static_cast<long long>(nc_) + ghost_owner_[g - n_]];
+    if (HostStage::pinned(host)) {
+      check(cudaMemcpy2DAsync(host, static_cast<size_t>(nc_) * sizeof(double), dev, per, per, 5,
+                              cudaMemcpyDeviceToHost, stream), "download");
+      check(cudaStreamSynchronize(stream), "download");
+    } else if (per < kRowsAtOnce && (per >= kRowsPinned || (++copies_out_ <= 2 && rows_host_ == nullptr))) {
+      // (pinned memory takes a millisecond or two to get: not for a handle's first copies)
+      check(cudaMemcpy2DAsync(host, static_cast<size_t>(nc_) * sizeof(double), dev, per, per, 5,
+                              cudaMemcpyDeviceToHost, stream), "download");
+      check(cudaStreamSynchronize(stream), "download");
+    } else if (per < kRowsAtOnce) {
+      // one copy into pinned memory of the handle's, then the rows (31 000 cells: 109 us; one 2-D copy
+      // into the caller's 271, a copy a component 336)
+      if (rows_host_ == nullptr)
+        check(cudaMallocHost(reinterpret_cast<void**>(&rows_host_), 5 * per), "cudaMallocHost");
+      check(cudaMemcpyAsync(rows_host_, dev, 5 * per, cudaMemcpyDeviceToHost, stream), "download");
+      check(cudaStreamSynchronize(stream), "download");
+      for (int k = 0; k < 5; ++k)
+        std::memcpy(host + k * static_cast<long long>(nc_), rows_host_ + k * static_cast<long long>(n_), per);
+    } else {
+      if (!out_stage_) out_stage_ = HostStage::of_device(1);
+      ++copies_out_;
+      for (int k = 0; k < 5; ++k)
+        check(out_stage_->to_host(host + k * static_cast<long long>(nc_), dev + k * static_cast<long long>(n_),
+                                  per, stream, copies_out_ > 1), "download");
+      check(cudaStreamSynchronize(stream), "download");
+    }
+    fill_images(host, zero_images);
   }
 
   // The primitives of the device state u_ into record buffer 0, where every step starts: a new
@@ -2960,9 +3002,7 @@ class Impl final : public Stepper {
     launch(k_store<P>, blocks(n_), kBlock, d_, static_cast<const double*>(stage_.as<double>()),
            prim_[1].as<C>());
     enqueue_residual(1);
-    copy_out(res_.as<double>(), res);
-    for (int k = 0; k < 5; ++k)
-      for (int g = n_; g < nc_; ++g) res[k * static_cast<long long>(nc_) + g] = 0.0;
+    copy_out(res_.as<double>(), res, true);
   }
 
   void evaluate(autan_euler_step_result* out) override {
@@ -3003,8 +3043,9 @@ class Impl final : public Stepper {
     need_ranks();
     if (ranked()) graph = false;  // the exchange callbacks run on the host between launches
     // Reset the step count so that the history holds this call's steps, and the fault word.
-    check(cudaMemsetAsync(&d_.ctl->step, 0, sizeof(long long), stream), "reset");
-    check(cudaMemsetAsync(&d_.ctl->fault, 0, sizeof(unsigned long long), stream), "reset");
+    // (step, dt and fault lie beside one another; a step sets dt anew)
+    static_assert(offsetof(Control, fault) == offsetof(Control, step) + 16, "one reset covers both");
+    check(cudaMemsetAsync(&d_.ctl->step, 0, 24, stream), "reset");
     const StepKey key{cfl, dt, local, rk};
     ready_walls();
     if (graph) {
@@ -3586,27 +3627,30 @@ class Impl final : public Stepper {
     launch_smem(kind, kernel, grid, block, 0, args...);
   }
 
+  // Launches of `kernel` with `smem` bytes of dynamic shared memory above 48 KB allowed: its
+  // limit raised to the device's opt-in maximum less its static shared memory, the same value from
+  // every handle and thread (a limit set to each launch's own size would race with another handle's
+  // launch of the same kernel at a larger size).
+  template <class K>
+  void allow_smem(K kernel, size_t smem) {
+    if (smem_optin_ == 0) {
+      int dev = 0;
+      check(cudaGetDevice(&dev), "device");
+      check(cudaDeviceGetAttribute(&smem_optin_, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "device");
+    }
+    cudaFuncAttributes fa{};
+    check(cudaFuncGetAttributes(&fa, kernel), "shared memory");
+    const long long limit = static_cast<long long>(smem_optin_) - static_cast<long long>(fa.sharedSizeBytes);
+    if (static_cast<long long>(smem) > limit) fail("E1200: shared memory above the device's limit");
+    check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(limit)),
+          "shared memory");
+  }
+
   template <class K, class... A>
   void launch_smem(int kind, K kernel, int grid, int block, size_t smem, A... args) {
     cudaEvent_t before = nullptr, after = nullptr;
     if (smem > 48 * 1024) {
-      // The kernel's dynamic shared-memory limit raised to the device's opt-in maximum less its
-      // static shared memory, the same value from every handle and thread: a limit set to each
-      // launch's own size would race with another handle's launch of the same kernel at a larger
-      // size.
-      if (smem_optin_ == 0) {
-        int dev = 0;
-        check(cudaGetDevice(&dev), "device");
-        check(cudaDeviceGetAttribute(&smem_optin_, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev),
-              "device");
-      }
-      cudaFuncAttributes fa{};
-      check(cudaFuncGetAttributes(&fa, kernel), "shared memory");
-      const long long limit =
-          static_cast<long long>(smem_optin_) - static_cast<long long>(fa.sharedSizeBytes);
-      if (static_cast<long long>(smem) > limit) fail("E1200: shared memory above the device's limit");
-      check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(limit)), "shared memory");
+      allow_smem(kernel, smem);
     }
     if (timing_) {
       check(cudaEventCreate(&before), "event");
@@ -3760,9 +3804,7 @@ class Impl final : public Stepper {
     prepare(u);
     enqueue_face_parts();
     if (res_faces != nullptr) {
-      copy_out(res_.as<double>(), res_faces);
-      for (int k = 0; k < 5; ++k)
-        for (int g = n_; g < nc_; ++g) res_faces[k * static_cast<long long>(nc_) + g] = 0.0;
+      copy_out(res_.as<double>(), res_faces, true);
     }
     if (face_flux != nullptr) {
       Buffer out(5ULL * nf_ * sizeof(double));
@@ -4127,7 +4169,7 @@ class Impl final : public Stepper {
           if constexpr (std::is_same_v<P, Fp32Acc64> && L) {
             if (tuning_.grad_mode == 4) launch_gradients_w<D>(d, cfl, loc);
             if (tuning_.grad_mode == 5) launch_gradients_ring<D>(d, cfl, loc);
-            if (tuning_.grad_mode != 6) return;
+            if (tuning_.grad_mode < 6) return;
           }
           // fp64, no limiter, or a mesh that fits no split blocks: the mode-0 form with two entries in flight
           if constexpr (sizeof(C) == 4)
@@ -4418,6 +4460,9 @@ class Impl final : public Stepper {
   bool chained_ = false;  // set around launches of kernels that wait for the previous one themselves
   bool step_tiles_ = false;  // set while enqueue_step records: its launches use the tiles
   Control* head_ = nullptr;  // pinned copy of the control's head
+  double* rows_host_ = nullptr;  // pinned rows of a small state on its way out
+  std::shared_ptr<HostStage> in_stage_, out_stage_;
+  int copies_in_ = 0, copies_out_ = 0;  // the handle's pageable state copies so far
   cudaStream_t side_ = nullptr;  // a step's norms, beside its later stages
   cudaEvent_t forked_ = nullptr, joined_ = nullptr;
   struct Timed {

@@ -17,6 +17,7 @@
 #include <stdio.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -26,6 +27,7 @@
 #include <vector>
 
 #include "autan_mlp.h"
+#include "host_stage.hpp"
 
 namespace autan_b200 {
 namespace mlp {
@@ -735,8 +737,7 @@ __global__ void __launch_bounds__(128) k_wall_distance(const double* tri, const 
     const int seen = at;
     float limit = 0.0f;
     auto set_limit = [&]() {
-      const float b = static_cast<float>(best) * 1.00001f;
-      limit = b * b * 1.00001f + 1e-37f;
+      limit = static_cast<float>(best) * 1.00003f + 1e-37f;
     };
     set_limit();
     // every node in order, a left-out one with all below it
@@ -765,7 +766,7 @@ __global__ void __launch_bounds__(128) k_wall_distance(const double* tri, const 
       }
     }
   }
-  out[i] = best;
+  out[i] = sqrt(best);
 }
 
 // ---------------------------------------------------------------- host
@@ -865,6 +866,11 @@ class Net {
   ~Net() {
     cudaStreamSynchronize(stream_);
     if (se_host_ != nullptr) cudaFreeHost(se_host_);
+    if (out_stream_ != nullptr) {
+      cudaStreamDestroy(out_stream_);
+      for (cudaEvent_t e : ring_done_)
+        if (e != nullptr) cudaEventDestroy(e);
+    }
     cudaStreamDestroy(stream_);
   }
 
@@ -897,8 +903,8 @@ class Net {
     n_data_ = n;
     x_.alloc(static_cast<size_t>(n) * inputs_ * 4);
     y_.alloc(static_cast<size_t>(n) * outputs_ * 4);
-    copy(x_, x, static_cast<size_t>(n) * inputs_ * 4);
-    copy(y_, y, static_cast<size_t>(n) * outputs_ * 4);
+    put(x_.p, x, static_cast<size_t>(n) * inputs_ * 4);
+    put(y_.p, y, static_cast<size_t>(n) * outputs_ * 4);
     sync();
   }
 
@@ -1100,49 +1106,117 @@ class Net {
   }
 
   void predict(const float* x, long long n, float* y, bool device_ptrs) {
-    const long long chunk = 1 << 18;
-    Buf xd, yd;
-    if (!device_ptrs) {
-      xd.alloc(static_cast<size_t>(n) * inputs_ * 4);
-      yd.alloc(static_cast<size_t>(n) * outputs_ * 4);
-      copy(xd, x, static_cast<size_t>(n) * inputs_ * 4);
+    if (device_ptrs) {
+      for (long long r0 = 0; r0 < n; r0 += kPredictChunk)
+        predict_rows(x + r0 * inputs_, static_cast<int>(std::min(kPredictChunk, n - r0)), y + r0 * outputs_);
+    } else if (++host_calls_, n <= kPredictPiece) {
+      ensure(px_, static_cast<size_t>(n) * inputs_ * 4);
+      ensure(py_, static_cast<size_t>(n) * outputs_ * 4);
+      put(px_.p, x, static_cast<size_t>(n) * inputs_ * 4);
+      predict_rows(px_.as<float>(), static_cast<int>(n), py_.as<float>());
+      get(y, py_.p, static_cast<size_t>(n) * outputs_ * 4, stream_);
+    } else {
+      predict_pieces(x, n, y);
     }
-    const float* xs = device_ptrs ? x : xd.as<float>();
-    float* ys = device_ptrs ? y : yd.as<float>();
-    const int L = static_cast<int>(layers_.size());
-    for (long long r0 = 0; r0 < n; r0 += chunk) {
-      const int rows = static_cast<int>(std::min(chunk, n - r0));
-      if (fused_) {
-        const int tiles = blocks(rows, 128);
-        fused_attrs();
-        fused::k_fused<false><<<std::min(tiles, sms_), fused::kThreads, fused::kSmem, stream_>>>(
-            lay_, xs + r0 * inputs_, nullptr, nullptr, rows, tiles, nullptr, nullptr, nullptr, 0,
-            nullptr, 0.0f, ys + r0 * outputs_, fault_.as<unsigned int>());
-        check(cudaGetLastError(), "fused predict");
-        continue;
-      }
-      ensure_work(rows);
-      launch_inputs(xs + r0 * inputs_, nullptr, rows);
-      forward(rows, false);
-      k_outputs<<<blocks(static_cast<long long>(rows) * outputs_, 256), 256, 0, stream_>>>(
-          zf(L - 1), layers_[L - 1].np, outputs_, rows, out_mean_.as<float>(), out_sd_.as<float>(),
-          ys + r0 * outputs_);
-      check(cudaGetLastError(), "outputs");
-    }
-    if (!device_ptrs)
-      check(cudaMemcpyAsync(y, yd.p, static_cast<size_t>(n) * outputs_ * 4, cudaMemcpyDeviceToHost, stream_),
-            "predict");
     sync();
+  }
+
+  // One launch (fused engine) or one pass of the layers over `rows` rows on the device.
+  void predict_rows(const float* xs, int rows, float* ys) {
+    const int L = static_cast<int>(layers_.size());
+    if (fused_) {
+      const int tiles = blocks(rows, 128);
+      fused_attrs();
+      fused::k_fused<false><<<std::min(tiles, sms_), fused::kThreads, fused::kSmem, stream_>>>(
+          lay_, xs, nullptr, nullptr, rows, tiles, nullptr, nullptr, nullptr, 0, nullptr, 0.0f, ys,
+          fault_.as<unsigned int>());
+      check(cudaGetLastError(), "fused predict");
+      return;
+    }
+    ensure_work(rows);
+    launch_inputs(xs, nullptr, rows);
+    forward(rows, false);
+    k_outputs<<<blocks(static_cast<long long>(rows) * outputs_, 256), 256, 0, stream_>>>(
+        zf(L - 1), layers_[L - 1].np, outputs_, rows, out_mean_.as<float>(), out_sd_.as<float>(), ys);
+    check(cudaGetLastError(), "outputs");
+  }
+
+  // Many host rows, in pieces through a ring of device buffers: this thread copies a piece's inputs in
+  // and launches it, a second one copies the predictions out, so that the inputs of a piece, the pass
+  // over the one before and the predictions of the one before that are under way together.
+  void predict_pieces(const float* x, long long n, float* y) {
+    const size_t xp = static_cast<size_t>(kPredictPiece) * inputs_, yp = static_cast<size_t>(kPredictPiece) * outputs_;
+    ensure(px_, kRing * xp * 4);
+    ensure(py_, kRing * yp * 4);
+    if (out_stream_ == nullptr) {
+      check(cudaStreamCreateWithFlags(&out_stream_, cudaStreamNonBlocking), "stream");
+      for (cudaEvent_t& e : ring_done_) check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+    }
+    const long long pieces = (n + kPredictPiece - 1) / kPredictPiece;
+    auto rows_of = [&](long long p) { return static_cast<int>(std::min(kPredictPiece, n - p * kPredictPiece)); };
+    std::atomic<long long> launched{0}, drained{0};
+    std::atomic<bool> stop{false};
+    std::exception_ptr failed;
+    get_stage();
+    auto drain = [&] {
+      try {
+        check(cudaSetDevice(device_), "cudaSetDevice");
+        for (long long p = 0; p < pieces; ++p) {
+          while (launched.load(std::memory_order_acquire) <= p) {
+            if (stop.load()) return;
+            std::this_thread::yield();
+          }
+          const int b = static_cast<int>(p % kRing);
+          check(cudaStreamWaitEvent(out_stream_, ring_done_[b], 0), "predict");
+          get(y + p * kPredictPiece * outputs_, py_.as<float>() + b * yp,
+              static_cast<size_t>(rows_of(p)) * outputs_ * 4, out_stream_);
+          check(cudaStreamSynchronize(out_stream_), "predict");  // (the caller's memory may be pinned)
+          drained.store(p + 1, std::memory_order_release);
+        }
+      } catch (...) {
+        failed = std::current_exception();
+        stop.store(true);
+      }
+    };
+    std::thread out(drain);
+    try {
+      for (long long p = 0; p < pieces && !stop.load(); ++p) {
+        while (p - drained.load(std::memory_order_acquire) >= kRing && !stop.load()) std::this_thread::yield();
+        if (stop.load()) break;
+        const int b = static_cast<int>(p % kRing);
+        float* xs = px_.as<float>() + b * xp;
+        put(xs, x + p * kPredictPiece * inputs_, static_cast<size_t>(rows_of(p)) * inputs_ * 4);
+        predict_rows(xs, rows_of(p), py_.as<float>() + b * yp);
+        check(cudaEventRecord(ring_done_[b], stream_), "predict");
+        launched.store(p + 1, std::memory_order_release);
+      }
+    } catch (...) {
+      stop.store(true);
+      out.join();
+      throw;
+    }
+    out.join();
+    if (failed) std::rethrow_exception(failed);
   }
 
   // One forward and backward pass on host rows, no update: the loss and the gradient.
   float gradient(const float* x, const float* y, int n, float* g) {
-    Buf xd(static_cast<size_t>(n) * inputs_ * 4), yd(static_cast<size_t>(n) * outputs_ * 4);
-    copy(xd, x, static_cast<size_t>(n) * inputs_ * 4);
-    copy(yd, y, static_cast<size_t>(n) * outputs_ * 4);
-    const float l = forward_backward(xd.as<float>(), yd.as<float>(), nullptr, n);
+    ensure(px_, static_cast<size_t>(n) * inputs_ * 4);
+    ensure(py_, static_cast<size_t>(n) * outputs_ * 4);
+    ++host_calls_;
+    put(px_.p, x, static_cast<size_t>(n) * inputs_ * 4);
+    put(py_.p, y, static_cast<size_t>(n) * outputs_ * 4);
+    if (!fused_) {
+      const float l = forward_backward(px_.as<float>(), py_.as<float>(), nullptr, n);
+      grad_to(g);
+      return l;
+    }
+    // the squared errors and the gradient come back behind one wait
+    fused_pass(px_.as<float>(), py_.as<float>(), nullptr, n, false, 0.0f, 0.0f, 0.0f);
+    std::vector<float> se(n);
+    check(cudaMemcpyAsync(se.data(), fse_.p, static_cast<size_t>(n) * 4, cudaMemcpyDeviceToHost, stream_), "loss");
     grad_to(g);
-    return l;
+    return loss_of(se.data(), n);
   }
 
   void grad_to(float* g) {
@@ -1267,13 +1341,25 @@ class Net {
   void ensure(Buf& b, size_t bytes) {
     if (b.n < bytes) b.alloc(bytes);
   }
+  // Rows between the caller's memory and the device (host_stage.hpp).
+  void put(void* dev, const void* host, size_t bytes) {
+    if (!in_stage_) in_stage_ = HostStage::of_device(0);
+    check(in_stage_->to_device(dev, host, bytes, stream_, host_calls_ > 1 || bytes >= (size_t(64) << 20)), "copy");
+  }
+  void get_stage() {
+    if (!out_stage_) out_stage_ = HostStage::of_device(1);
+  }
+  void get(void* host, const void* dev, size_t bytes, cudaStream_t s) {
+    get_stage();
+    check(out_stage_->to_host(host, dev, bytes, s, host_calls_ > 1), "copy");
+  }
   void copy(Buf& b, const void* host, size_t bytes) {
     check(cudaMemcpyAsync(b.p, host, bytes, cudaMemcpyHostToDevice, stream_), "copy");
   }
   void sync() {
-    check(cudaStreamSynchronize(stream_), "sync");
     unsigned int f = 0;
-    check(cudaMemcpy(&f, fault_.p, sizeof(f), cudaMemcpyDeviceToHost), "fault");
+    check(cudaMemcpyAsync(&f, fault_.p, sizeof(f), cudaMemcpyDeviceToHost, stream_), "fault");
+    check(cudaStreamSynchronize(stream_), "sync");
     if (f != 0) {
       // reported once: the word is cleared so that the handle's next call starts clean
       check(cudaMemset(fault_.p, 0, sizeof(unsigned int)), "fault");
@@ -1320,6 +1406,15 @@ class Net {
   int sms_ = 148;
   fused::Layout lay_{};
   Buf zbuf_, atbuf_, fpartial_, fse_;
+  // Rows of host calls on the device: the largest gradient call's, or the ring of predict_pieces
+  // (kRing x 2^17 rows at most), kept for the next call.
+  static constexpr long long kPredictChunk = 1 << 18, kPredictPiece = 1 << 17;
+  static constexpr int kRing = 3;
+  Buf px_, py_;
+  cudaStream_t out_stream_ = nullptr;
+  cudaEvent_t ring_done_[kRing] = {};
+  std::shared_ptr<HostStage> in_stage_, out_stage_;
+  int host_calls_ = 0;  // calls with host rows so far
   std::vector<std::unique_ptr<Buf>> wk_img_, wt_img_;
   Buf params_, grad_, m_, v_, in_mean_, in_sd_, out_mean_, out_sd_, x_, y_, idx_, fault_;
   float* se_host_ = nullptr;  // pinned: an epoch's per-row squared errors
@@ -1480,7 +1575,8 @@ int autan_wall_distance(const double* triangles, const int64_t* tri_offsets, con
     const size_t o_tri = take(static_cast<size_t>(std::max<int64_t>(nt, 1)) * 72),
                  o_tree = take(static_cast<size_t>(n_cases) * sizeof(CaseTree)),
                  o_node = take(static_cast<size_t>(std::max<int64_t>(n_nodes, 1)) * 32),
-                 o_off = take((static_cast<size_t>(n_cases) + 1) * 8), o_pts = take(np * 24), o_out = take(np * 8);
+                 o_off = take((static_cast<size_t>(n_cases) + 1) * 8),
+                 o_pts = take(np * 24), o_out = take(np * 8);
     Buf mem(total);
     unsigned char* m = mem.as<unsigned char>();
     auto* tri = reinterpret_cast<double*>(m + o_tri);
@@ -1492,7 +1588,14 @@ int autan_wall_distance(const double* triangles, const int64_t* tri_offsets, con
     if (nt > 0) check(cudaMemcpy(tri, triangles, nt * 9 * 8, cudaMemcpyHostToDevice), "copy");
     check(cudaMemcpy(tree, trees.data(), trees.size() * sizeof(CaseTree), cudaMemcpyHostToDevice), "copy");
     check(cudaMemcpy(off, point_offsets, (n_cases + 1) * 8, cudaMemcpyHostToDevice), "copy");
-    check(cudaMemcpy(pts, points, n_points * 3 * 8, cudaMemcpyHostToDevice), "copy");
+    // (the pinned slots are worth their allocation from some tens of megabytes; there is no handle here
+    // that would keep them from one call to the next)
+    const bool staged = n_points > (1 << 21);
+    if (staged)
+      check(autan_b200::HostStage::of_device(0)->to_device(pts, points, static_cast<size_t>(n_points) * 24, nullptr,
+                                                       true), "copy");
+    else
+      check(cudaMemcpy(pts, points, static_cast<size_t>(n_points) * 24, cudaMemcpyHostToDevice), "copy");
     // at most 65535 cases in the grid's y: more go in further launches
     for (int level = 0; level < levels; ++level)
       for (int k0 = 0; k0 < n_cases; k0 += 65535) {
@@ -1502,7 +1605,11 @@ int autan_wall_distance(const double* triangles, const int64_t* tri_offsets, con
       }
     k_wall_distance<<<blocks(n_points, 128), 128>>>(tri, tree, node, off, n_cases, pts, n_points, out);
     check(cudaGetLastError(), "wall distance");
-    check(cudaMemcpy(distance, out, n_points * 8, cudaMemcpyDeviceToHost), "copy");
+    if (staged)
+      check(autan_b200::HostStage::of_device(1)->to_host(distance, out, static_cast<size_t>(n_points) * 8, nullptr,
+                                                     true), "copy");
+    check(staged ? cudaStreamSynchronize(nullptr)
+                 : cudaMemcpy(distance, out, static_cast<size_t>(n_points) * 8, cudaMemcpyDeviceToHost), "copy");
   });
 }
 

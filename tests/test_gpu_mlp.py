@@ -140,6 +140,22 @@ def test_engines_agree(rows):
         assert np.linalg.norm(g0 - g1) <= 2e-2 * np.linalg.norm(g0)
 
 
+@pytest.mark.parametrize("engine", [0, 2])
+def test_prediction_in_pieces(engine):
+    """More rows than one piece (2^17) and than the ring of pieces holds, a ragged last one: the rows of
+    one call equal those of calls of their own, whatever they share a piece with."""
+    n = 4 * 131072 + 77
+    x, y = data(20000, seed=13)
+    x = np.concatenate([x] * (n // 20000 + 1))[:n]
+    x[::3] *= 0.5
+    net = MLP(seed=14)
+    net.set_engine(engine)
+    net.set_scaling(*scaling(x[:20000], y))
+    got = net.predict(x)
+    for a, b in ((0, 1000), (131072 - 300, 131072 + 300), (400000, 400128), (n - 77, n)):
+        assert np.array_equal(got[a:b], net.predict(x[a:b]))
+
+
 def test_fused_engine_is_the_default_and_deterministic():
     """Width 128: the fused engine unless another is chosen; two passes give the same bits (the
     CTAs' partials are summed in a fixed order); other widths refuse it."""

@@ -315,6 +315,21 @@ def test_block_forms_are_bit_identical(build, precision):
             assert bits_equal(a, b), (tuning, graph, between)
 
 
+@pytest.mark.parametrize("n", [(17, 15, 3), (400, 340, 1), (1060, 1000, 1)], ids=["765", "136k", "1060k"])
+def test_states_come_back_as_they_went(n):
+    """A state to the device and back three times from pageable memory: rows through the handle's pinned
+    memory (small states, from the third copy), one copy of five rows (middle), the shared pinned slots
+    (8 MB a component and more, from the second); images of owned cells with their owner's values."""
+    case = cases.vortex_hex(*n, steps=1)
+    rng = np.random.default_rng(1)
+    with EulerDevice(case.mesh, case.scheme, case.bc_kind, case.bc_data) as dev:
+        for _ in range(4):
+            u = case.u0 * (1.0 + 1e-3 * rng.standard_normal(case.u0.shape))
+            u[:, case.mesh.n_owned_cells:] = u[:, case.mesh.ghost_owner]
+            dev.upload(u)
+            assert bits_equal(dev.download(), u)
+
+
 def test_autotune_leaves_the_solution_unchanged():
     case = cases.vortex_tets(20, 20, 6, steps=3, precision="fp32+acc64")
     a, *_ = run_device(case, case.steps)

@@ -579,9 +579,11 @@ __device__ __forceinline__ V3 axpy(V3 a, double s, V3 d) {
   return {a.x + s * d.x, a.y + s * d.y, a.z + s * d.z};
 }
 
-// Distance from p to triangle (a, b, c): the closest point by the Voronoi regions of the
-// triangle's vertices, edges and face (Ericson, Real-Time Collision Detection, 2005, sec. 5.1.5).
-__device__ double point_triangle(V3 p, V3 a, V3 b, V3 c) {
+// Squared distance from p to triangle (a, b, c): the closest point by the Voronoi regions of the
+// triangle's vertices, edges and face (Ericson, Real-Time Collision Detection, 2005, sec. 5.1.5). The
+// least of the squares has the least root (the rounded square root is monotonic), so that one root a
+// point is enough.
+__device__ double point_triangle2(V3 p, V3 a, V3 b, V3 c) {
   const V3 ab = sub3(b, a), ac = sub3(c, a), ap = sub3(p, a);
   const double d1 = dot(ab, ap), d2 = dot(ac, ap);
   V3 q;
@@ -611,7 +613,7 @@ __device__ double point_triangle(V3 p, V3 a, V3 b, V3 c) {
     }
   }
   const V3 d = sub3(p, q);
-  return sqrt(dot(d, d));
+  return dot(d, d);
 }
 
 // A tree of boxes over each case's triangles: leaves of kLeaf consecutive triangles (a wall's fan
@@ -620,7 +622,7 @@ __device__ double point_triangle(V3 p, V3 a, V3 b, V3 c) {
 // down to one leaf first (a good bound), then through the tree leaving out the boxes that are farther
 // than the least distance so far, so it forms the distances of a few tens of triangles instead of all.
 // The triangles that are left out could not be the least: boxes and comparisons keep a margin (below)
-// far above the rounding of point_triangle, whose values the minimum is still taken over.
+// far above the rounding of point_triangle2, whose values the minimum is still taken over.
 constexpr int kLeaf = 4;
 constexpr int kFan = 8;
 constexpr int kTreeLevels = 24;
@@ -683,7 +685,7 @@ __global__ void k_wall_nodes(const double* tri, const CaseTree* trees, int level
   }
 }
 
-// The distance of every point to its case's triangles, exact: the least of point_triangle's values.
+// The distance of every point to its case's triangles, exact: the root of point_triangle2's least value.
 // Bound by the FP64 work of the triangles a point still meets and the divergence of the searches:
 // 229 000 cells of four channels against 4 000 to 9 000 triangles each, 6.42 ms over every triangle,
 // 0.77 ms through the tree.
@@ -705,7 +707,7 @@ __global__ void __launch_bounds__(128) k_wall_distance(const double* tri, const 
   auto leaf = [&](int l) {
     for (int t = l * kLeaf; t < min(T.n, (l + 1) * kLeaf); ++t) {
       const double* q = tri + 9 * (T.tri0 + t);
-      const double d = point_triangle(p, {q[0], q[1], q[2]}, {q[3], q[4], q[5]}, {q[6], q[7], q[8]});
+      const double d = point_triangle2(p, {q[0], q[1], q[2]}, {q[3], q[4], q[5]}, {q[6], q[7], q[8]});
       if (d < best) best = d;
     }
   };

@@ -410,12 +410,19 @@ def parse_triple(text: str) -> tuple[int, int, int]:
 # ------------------------------------------------------------------ arms
 
 
+NO_REFERENCE = "the reference's set-up library (oracle/_ref) is not built: its sources are not here"
+
+
 def run_reference(args, rank: int, world: int) -> None:
     if rank != 0:
         return
     threads = args.cpu_threads or host_threads()
-    rate, sample, cores = cpu_throughput(args.steps, max(1, min(args.warmup, 1)), threads,
-                                         args.workload)  # fmt: skip
+    try:
+        rate, sample, cores = cpu_throughput(args.steps, max(1, min(args.warmup, 1)), threads,
+                                             args.workload)  # fmt: skip
+    except OSError:
+        print(json.dumps({"impl": "reference", "unavailable": NO_REFERENCE}), flush=True)
+        return
     line = {
         "impl": "reference",
         "metric": "cell-iterations/s",
@@ -850,10 +857,13 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
         dist.destroy_process_group()
     if rank == 0:
         if world == 1 and not args.no_cpu:
-            rate, sample, cores = cpu_throughput(2, 1, args.cpu_threads or host_threads(),
-                                                 args.workload, min_seconds=10.0)  # fmt: skip
-            line["cpu_baseline"] = {"value": rate, "unit": "cell-iterations/s", "cores": cores,
-                                    "kind": "port", "sample": sample}  # fmt: skip
+            try:
+                rate, sample, cores = cpu_throughput(2, 1, args.cpu_threads or host_threads(),
+                                                     args.workload, min_seconds=10.0)  # fmt: skip
+                line["cpu_baseline"] = {"value": rate, "unit": "cell-iterations/s", "cores": cores,
+                                        "kind": "port", "sample": sample}  # fmt: skip
+            except OSError:  # oracle/_ref is built only where the reference's sources are
+                line["cpu_baseline"] = {"unavailable": NO_REFERENCE}
         print(json.dumps(line), flush=True)
 
 

@@ -27,7 +27,12 @@
 //   k_faces            per cell: every face flux of the cell recomputed (gather-recompute: no float
 //                      atomics, no face scratch), summed in face order from the source term, then
 //                      the RK stage update in FP64 and the next stage's primitives.
-// Per step: the exact-sum residual norms of stage 0. A step is captured in one CUDA graph.
+// Small and medium meshes take blocks of consecutive cells instead (cell_blocks.cuh, face_blocks.cuh):
+//   k_gradients_split  five threads a cell, the block's rows and neighbour records in shared memory;
+//   k_faces_block      the block's face fluxes in shared memory, their sums, the RK stage and the next
+//                      stage's boundary states.
+// Per step: the exact-sum residual norms of stage 0, on a side stream beside the later stages. A step
+// is captured in one CUDA graph.
 #include <cuda_runtime.h>
 
 #include <algorithm>

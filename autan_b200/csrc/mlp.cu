@@ -687,8 +687,8 @@ __global__ void k_wall_nodes(const double* tri, const CaseTree* trees, int level
 
 // The distance of every point to its case's triangles, exact: the root of point_triangle2's least value.
 // Bound by the FP64 work of the triangles a point still meets and the divergence of the searches:
-// 229 000 cells of four channels against 4 000 to 9 000 triangles each, 6.42 ms over every triangle,
-// 0.77 ms through the tree.
+// 183 000 cells of four channels against 4 000 to 8 000 triangles each, 6.42 ms over every triangle,
+// 0.69 ms through the tree.
 __global__ void __launch_bounds__(128) k_wall_distance(const double* tri, const CaseTree* trees,
                                                        const float4* nodes, const int64_t* pt_off,
                                                        int n_cases, const double* pts, long long n,

@@ -3726,6 +3726,7 @@ class Impl final : public Stepper {
       FacePlan& p = *block_faces();
       const int bs = tuning_.face_block;
       const bool some = repacked() && p.n_active >= 0;
+      if (some && p.n_active == 0) return;  // every case has stopped
       // first order: only the next step's spectral radius reads boundary states
       const bool walls = carries_walls() && (second_ || last);
       FaceBlocks<P> g{p.first.template as<int>(), p.bfirst.template as<int>(),
@@ -3733,7 +3734,7 @@ class Impl final : public Stepper {
                       p.bface.template as<int>(), p.inc.template as<uint2>(),
                       p.inc_start.template as<int>(), walls ? p.wfirst.template as<int>() : nullptr,
                       p.walls.template as<int>(), some ? p.active.template as<int>() : nullptr, bs};
-      const int nblk = some ? std::max(p.n_active, 1) : blocks(n_, bs);
+      const int nblk = some ? p.n_active : blocks(n_, bs);
       dispatch_faces([&](auto flux, auto planar, auto second) {
         constexpr int F = decltype(flux)::value;
         constexpr bool PL = decltype(planar)::value, SE = decltype(second)::value;
@@ -4158,9 +4159,10 @@ class Impl final : public Stepper {
           const GradPlan& g = *split_plan();
           const int cells = std::min(bs, kSplitCells);
           const bool some = repacked() && g.n_active >= 0;
+          if (some && g.n_active == 0) return;  // every case has stopped
           GradBlocks<P> gb{g.off.template as<int>(), g.list.template as<int>(), g.st.template as<C>(),
                            g.inc.template as<C>(), some ? g.active.template as<int>() : nullptr};
-          const int nblk = some ? std::max(g.n_active, 1) : blocks(n_, cells);
+          const int nblk = some ? g.n_active : blocks(n_, cells);
           Chain chain(chained_);
           launch_smem(kGradients, k_gradients_split<P, L, D>, nblk, kSplit * cells,
                       grad_split_bytes<C>(g.shape, cells), d, gb, g.shape, cfl, loc);

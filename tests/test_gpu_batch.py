@@ -83,6 +83,30 @@ def test_stopped_case_is_unchanged_and_the_others_match_their_own_runs():
         assert bits_equal(u[:, c0:c1], uk)
 
 
+@pytest.mark.parametrize("blocks", [True, False], ids=["blocks", "store-gather"])
+@pytest.mark.parametrize("graph", [True, False])
+def test_every_case_stopped_leaves_the_state_and_the_handle_usable(blocks, graph):
+    """No active case: no block of cells has work (their list is empty), the state comes back bit for
+    bit; with the cases active again the steps are a fresh handle's."""
+    b = small_batch()
+
+    def run(stop_first):
+        with device_of(b) as dev:
+            if not blocks:
+                dev.set_tuning(grad_mode=0, grad_chunk=2, grad_block=64, face_mode=1, face_block=64,
+                               gather_block=128)  # fmt: skip
+            if stop_first:
+                dev.set_active([0, 0, 0])
+                dev.step(cfl=b.cfl, rk=3, n_steps=2, local=True, graph=graph)
+                assert bits_equal(dev.download(), b.u0)
+                dev.set_active([1, 1, 1])
+            dev.step(cfl=b.cfl, rk=3, n_steps=3, local=True, graph=graph)
+            return dev.download(), dev.case_history(3)
+
+    for a, w in zip(run(True), run(False)):
+        assert bits_equal(a, w)
+
+
 def test_batched_march_converges_each_case_at_its_own_iteration():
     b = small_batch(cells=(300, 1500), n=4, seed=5)
     with device_of(b) as dev:

@@ -55,6 +55,7 @@
 #include "convergence.hpp"
 #include "exact_sum.cuh"
 #include "host_stage.hpp"
+#include "tuning_trials.hpp"
 
 namespace autan_b200 {
 
@@ -3184,57 +3185,40 @@ class Impl final : public Stepper {
       return (kind < 0 ? total : picked) / trial_steps;
     };
     Tuning best = tuning_;
+    const TrialScope scope = trial_scope(
+        second_, n_, [&](bool mine) { return any_rank(mine); },
+        [&](int block) { return grad_plan(block) != nullptr; },
+        [&](int block) { return face_plan(block) != nullptr; });
     if (second_) {
       double best_ms = 1e300;
-      Tuning keep = best;
-      auto trial = [&](int mode, int chunk, int block, int minb) {
+      const Tuning keep = best;
+      for (const GradTrial& g : grad_trials(scope, sizeof(C) == 4 && limiter_)) {
         Tuning t = keep;
-        t.grad_mode = mode;
-        t.grad_chunk = chunk;
-        t.grad_block = block;
-        t.grad_minb = minb;
+        t.grad_mode = g.mode;
+        t.grad_chunk = g.chunk;
+        t.grad_block = g.block;
+        t.grad_minb = g.minb;
         const double ms = measure(t, kGradients);
         if (ms < best_ms) {
           best_ms = ms;
           best = t;
         }
-      };
-      // (the pipelined, ring and widening forms were never the fastest on any measured case: they stay
-      // open to set_tuning and are not tried)
-      for (int block : {64, 128}) {
-        for (int chunk : {1, 2, 4}) trial(0, chunk, block, 7);
-        for (int chunk : {4, 8}) trial(1, chunk, block, 7);
       }
-      if (sizeof(C) == 4 && limiter_)
-        for (int minb : {7, 6, 5}) trial(4, minb == 5 ? 4 : 2, 128, minb);
-      // the split form, where the mesh is small enough for it to win
-      if (n_ <= 148 * 2048)
-        for (int block : {32, kSplitCells})
-          if (grad_plan(block) != nullptr) trial(6, 2, block, 7);
     }
     {
       double best_ms = 1e300;
-      Tuning keep = best;
-      auto trial = [&](int mode, int block, int gather) {
+      const Tuning keep = best;
+      for (const FaceTrial& f : face_trials(scope, n_cases_ > 0)) {
         Tuning t = keep;
-        t.face_mode = mode;
-        t.face_block = block;
-        t.gather_block = gather;
+        t.face_mode = f.mode;
+        t.face_block = f.block;
+        t.gather_block = f.threads;
         const double ms = measure(t, kFaces);
         if (ms < best_ms) {
           best_ms = ms;
           best = t;
         }
-      };
-      const bool small = n_ <= 148 * 512;
-      if (small) trial(0, 64, 256);
-      for (int mode : {1, 2})
-        for (int block : {64, 128})
-          for (int gather : {128, 256})
-            if (mode == 1 || n_cases_ == 0) trial(mode, block, gather);  // mode 2 with cases: as mode 1
-      for (int block : {32, 64, 128})
-        for (int threads : {block, 2 * block, 4 * block, 8 * block})
-          if (threads <= 256 && (block == 128 || small) && face_plan(block) != nullptr) trial(3, block, threads);
+      }
     }
     // Whole steps as they run (their graph; the launches of a step overlap, which the sums above do not
     // see): the choices found against a new handle's.

@@ -324,3 +324,56 @@ def test_partitioned_march_takes_the_whole_mesh_steps(bad):
                                                                    ref["converged"])  # fmt: skip
         assert same_bits(r["last"], ref["last"])
         assert r["invalid_cell"] == ref["invalid_cell"]
+
+
+def test_autotune_of_unequal_ranks_makes_the_same_exchanges():
+    """Two ranks on either side of the tuner's size limits (90 000 and 16 000 cells) tune together: the
+    same exchanges and reductions on both, the solution unchanged, and the next steps the whole mesh's."""
+    case = K.bump_channel(60, 40, 40, steps=2)
+    m = case.mesh
+    cut = int(0.85 * m.n_owned_cells)
+    parts = (np.arange(m.n_owned_cells) >= cut).astype(np.int32)
+    assert cut > 148 * 512 > m.n_owned_cells - cut
+    weights = m.gradient_weights(case.bc_kind)
+    u0 = perturbed(case, 1e-3, 8)
+    ref = whole(case, weights, u0, 2)
+    ps = PT.extract_partitions(m, weights, parts)
+
+    class Counting(PT.ThreadRanks):
+        made = [0, 0]
+
+        def exchange(self, member, *args):
+            self.made[member.part.rank] += 1
+            super().exchange(member, *args)
+
+        def reduce(self, member, *args):
+            self.made[member.part.rank] += 1
+            super().reduce(member, *args)
+
+    ranks = Counting(2, timeout=60)
+    members = [PT.PartitionedEuler(p, case.scheme, ranks, case.bc_kind, case.bc_data) for p in ps]
+    out, errors = [None, None], []
+
+    def run(i):
+        try:
+            members[i].upload(u0)
+            members[i].autotune(case.cfl, 0.0, case.local, case.rk, 1)
+            made = ranks.made[i]
+            members[i].step(case.cfl, 0.0, case.local, case.rk, 2)
+            out[i] = (made, members[i].history(2), members[i].download())
+        except BaseException as e:  # noqa: BLE001 (reported below)
+            errors.append(e)
+            ranks.barrier.abort()
+
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(timeout=600)
+    for mb in members:
+        mb.close()
+    assert not errors, errors
+    assert out[0][0] == out[1][0] > 100
+    for _, (rms, dt), _ in out:
+        assert same_bits(rms, ref[2]) and same_bits(dt, ref[3])
+    assert same_bits(PT.gather_state(ps, [o[2] for o in out], m.n_owned_cells), ref[0])

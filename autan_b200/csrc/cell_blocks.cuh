@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(kSplit * kSplitCells, 4)
     if (faces) bulk_to_shared(fr, g.inc + 4LL * i0, row * nf, &bar);
   }
   dependents_may_start();
-  const int z = previous_done();
+  previous_done();
   // the block's records: its own cells', then the listed ones'
   auto put = [&](int i, const C* w) {
 #pragma unroll
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(kSplit * kSplitCells, 4)
       if (i >= nb || i < own) {
         const int x = i < nb ? b * nb + i : __ldg(g.list + n0 + i - nb);
         C u[5];
-        load5<P>(d.prim + static_cast<long long>(x + z) * kPrimW, u);
+        load5<P, true>(d.prim + static_cast<long long>(x) * kPrimW, u);
         put(i, u);
       }
     }

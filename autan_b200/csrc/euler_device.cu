@@ -197,16 +197,15 @@ __device__ __forceinline__ int index_of(double x) {
 // Programmatic dependent launches (a step's chain of launches): a kernel lets the next one's blocks
 // start beside its own as soon as all of its blocks have, and itself waits for the previous one's end
 // before it reads or writes anything that a launch of the step writes; what it reads before (offsets,
-// rows, face records) no launch writes. previous_done returns 0: an index that a read through the
-// non-coherent path goes by takes it as a summand, so that the read cannot be moved before the wait.
-// Without the launch attribute both do nothing.
+// rows, face records) no launch writes. What launches write (primitives, reconstruction, boundary
+// states) such a kernel reads with ordinary loads after the wait (the MUT forms below), never through
+// the non-coherent path: that one is for data that nothing writes while the kernel is resident, and up
+// to three launches of a chain are resident at once. Without the launch attribute both do nothing.
 __device__ __forceinline__ void dependents_may_start() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-__device__ __forceinline__ int previous_done() {
-  int z;
-  asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, 0;" : "=r"(z) : : "memory");
-  return z;
+__device__ __forceinline__ void previous_done() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 template <class C>
@@ -220,17 +219,33 @@ template <class P>
 constexpr bool kFaceA32 = (kFace * sizeof(typename P::C)) % 32 == 0;
 
 // 32-byte vector loads and stores (the 256-bit ld / st of sm_100): one L1 wavefront per lane
-// where two 16-byte vectors take two. The address must be 32-byte aligned.
+// where two 16-byte vectors take two. The address must be 32-byte aligned. MUT: an ordinary load
+// (volatile: it stays after the wait for the previous launch), else the non-coherent path.
+template <bool MUT = false>
 __device__ __forceinline__ void ld32(const float* p, float* o) {
-  asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-      : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]), "=f"(o[6]),
-        "=f"(o[7])
-      : "l"(p));
+  if constexpr (MUT) {
+    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]),
+                   "=f"(o[6]), "=f"(o[7])
+                 : "l"(p));
+  } else {
+    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]), "=f"(o[6]),
+          "=f"(o[7])
+        : "l"(p));
+  }
 }
+template <bool MUT = false>
 __device__ __forceinline__ void ld32(const double* p, double* o) {
-  asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];"
-      : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3])
-      : "l"(p));
+  if constexpr (MUT) {
+    asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
+                 : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3])
+                 : "l"(p));
+  } else {
+    asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];"
+        : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3])
+        : "l"(p));
+  }
 }
 // L2 eviction priority (createpolicy): data a launch reads once marked first out, so that it does
 // not push the records many threads read out of L2.
@@ -261,14 +276,14 @@ __device__ __forceinline__ void st32(double* p, const double* v) {
 
 // Vector loads of a record's words [w, w + count), count a multiple of the 16-byte vector width:
 // with A32 (base + w 32-byte aligned) 32-byte vectors first, then 16-byte ones.
-template <class P, bool A32 = false>
+template <class P, bool A32 = false, bool MUT = false>
 __device__ __forceinline__ void load_words(const typename P::C* base, int w, int count,
                                            typename P::C* out) {
   using V = typename P::V;
   constexpr int kW32 = 32 / static_cast<int>(sizeof(typename P::C));
   if constexpr (A32) {
 #pragma unroll
-    for (int q = 0; q < count / kW32; ++q) ld32(base + w + kW32 * q, out + kW32 * q);
+    for (int q = 0; q < count / kW32; ++q) ld32<MUT>(base + w + kW32 * q, out + kW32 * q);
     const int done = (count / kW32) * kW32;
     base += done;
     out += done;
@@ -277,7 +292,9 @@ __device__ __forceinline__ void load_words(const typename P::C* base, int w, int
   const V* v = reinterpret_cast<const V*>(base + w);
 #pragma unroll
   for (int q = 0; q < count / P::kVec; ++q) {
-    const V x = __ldg(v + q);
+    V x;
+    if constexpr (MUT) x = v[q];
+    else x = __ldg(v + q);
     if constexpr (P::kVec == 4) {
       out[4 * q] = x.x;
       out[4 * q + 1] = x.y;
@@ -321,10 +338,10 @@ __device__ __forceinline__ void store_words(typename P::C* base, int w, int coun
 }
 
 // The primitives of cell c (words 0-4 of its primitive record).
-template <class P>
+template <class P, bool MUT = false>
 __device__ __forceinline__ void load_prim(const typename P::C* prim, int c, typename P::C* w) {
   typename P::C t[8];
-  load_words<P, true>(prim + static_cast<long long>(c) * kPrimW, 0, 8, t);
+  load_words<P, true, MUT>(prim + static_cast<long long>(c) * kPrimW, 0, 8, t);
 #pragma unroll
   for (int k = 0; k < 5; ++k) w[k] = t[k];
 }
@@ -332,14 +349,14 @@ __device__ __forceinline__ void load_prim(const typename P::C* prim, int c, type
 // Primitives, limiter and gradient of cell c: its primitive record and its word group of each of
 // the reconstruction array's groups (cell-contiguous within a group, so that the records of
 // consecutive cells share cache lines).
-template <class P>
+template <class P, bool MUT = false>
 __device__ __forceinline__ void load_recon(const Dev<P>& d, int c, typename P::C* w,
                                            typename P::C* phi, typename P::C* g) {
   typename P::C t[kRecon], q[8];
-  load_words<P, true>(d.prim + static_cast<long long>(c) * kPrimW, 0, 8, q);
+  load_words<P, true, MUT>(d.prim + static_cast<long long>(c) * kPrimW, 0, 8, q);
 #pragma unroll
   for (int k = 0; k < kRecon / kGroup; ++k)
-    load_words<P, true>(d.recon + k * d.rstride + static_cast<long long>(c) * kGroup, 0, kGroup,
+    load_words<P, true, MUT>(d.recon + k * d.rstride + static_cast<long long>(c) * kGroup, 0, kGroup,
                         t + kGroup * k);
 #pragma unroll
   for (int k = 0; k < 5; ++k) w[k] = q[k];
@@ -513,12 +530,12 @@ __device__ __forceinline__ double cell_time_step(const Dev<P>& d, int c, const t
       const int f = code >> 1;
       load_words<P, kFaceA32<P>>(d.face + static_cast<long long>(f) * kFace, 0, kFace, rec);
       const int o = (code & 1) ? index_of(rec[7]) : index_of(rec[11]);
-      load_prim<P>(d.prim, o, wn);
+      load_prim<P, true>(d.prim, o, wn);
     } else {
       const int b = -code - 1;
       load_words<P>(d.bface + static_cast<long long>(b) * kBface, 0, 4, rec);
       C t[8];
-      load_words<P, true>(d.prim_b + static_cast<long long>(b) * kPrimB, 0, 8, t);
+      load_words<P, true, true>(d.prim_b + static_cast<long long>(b) * kPrimB, 0, 8, t);
 #pragma unroll
       for (int k = 0; k < 5; ++k) wn[k] = t[k];
     }
@@ -530,19 +547,20 @@ __device__ __forceinline__ double cell_time_step(const Dev<P>& d, int c, const t
 
 // The primitives of a cell (words 0-4), of a boundary face's state or of a face's flux, five
 // values only; src is 32-byte aligned (record, prim_b and flux strides are multiples of 32 bytes).
-template <class P>
+template <class P, bool MUT = false>
 __device__ __forceinline__ void load5(const typename P::C* src, typename P::C* w) {
   if constexpr (P::kVec == 4) {
     float t[8];
-    ld32(src, t);
+    ld32<MUT>(src, t);
 #pragma unroll
     for (int k = 0; k < 5; ++k) w[k] = t[k];
   } else {
     double t[4];
-    ld32(src, t);
+    ld32<MUT>(src, t);
 #pragma unroll
     for (int k = 0; k < 4; ++k) w[k] = t[k];
-    w[4] = __ldg(src + 4);
+    if constexpr (MUT) w[4] = src[4];
+    else w[4] = __ldg(src + 4);
   }
 }
 
@@ -1555,12 +1573,10 @@ __global__ void __launch_bounds__(256) k_spectral(Dev<P> d, double cfl, int loca
   const bool live = c >= 0 && c < d.n && cell_active(d, c);
   double dt = 0.0;
   dependents_may_start();
-  const int z = previous_done();
-  d.prim += z;
-  d.prim_b += z;
+  previous_done();
   if (live) {
     C wc[5];
-    load_prim<P>(d.prim, c, wc);
+    load_prim<P, true>(d.prim, c, wc);
     dt = cell_time_step(d, c, wc, cfl);
     if (local && d.dt_local != nullptr) d.dt_local[c] = dt;
     if (dt_out != nullptr) dt_out[c] = dt;
@@ -1573,14 +1589,14 @@ enum Mode : int { kResidual = 0, kRk3 = 1, kRk4 = 2, kFaceParts = 3 };
 
 // The reconstruction data of a cell: primitives, limiter and gradient (zero gradient and limiter
 // for the first-order scheme).
-template <class P, bool SECOND>
+template <class P, bool SECOND, bool MUT = false>
 __device__ __forceinline__ void cell_recon(const Dev<P>& d, int c, typename P::C* w,
                                            typename P::C* phi, typename P::C* g) {
   using C = typename P::C;
   if constexpr (SECOND) {
-    load_recon<P>(d, c, w, phi, g);
+    load_recon<P, MUT>(d, c, w, phi, g);
   } else {
-    load5<P>(d.prim + static_cast<long long>(c) * kPrimW, w);
+    load5<P, MUT>(d.prim + static_cast<long long>(c) * kPrimW, w);
 #pragma unroll
     for (int k = 0; k < 15; ++k) g[k] = C(0.0);
 #pragma unroll

@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(256, (kFaceBlockMin<P, PLANAR, SECOND>))
     if (il > 0) places = __ldg(inc);
   }
   dependents_may_start();
-  const int z = previous_done();
+  previous_done();
   for (int i = t; i < nf + nbf; i += nt) {
     C out[5];
     if (i < nf) {
@@ -136,8 +136,8 @@ __global__ void __launch_bounds__(256, (kFaceBlockMin<P, PLANAR, SECOND>))
         }
       }
       if (!cell_active(d, index_of(fr[7]))) continue;
-      cell_recon<P, SECOND>(d, index_of(fr[7]) + z, wl, pl, gl);
-      cell_recon<P, SECOND>(d, index_of(fr[11]) + z, wr, pr, gr);
+      cell_recon<P, SECOND, true>(d, index_of(fr[7]), wl, pl, gl);
+      cell_recon<P, SECOND, true>(d, index_of(fr[11]), wr, pr, gr);
       const int f = PLANAR ? 0 : __ldg(g.face + f0 + i);
       interior_flux<P, FLUX, PLANAR>(d, f, fr, wl, gl, pl, wr, gr, pr, out);
     } else {
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(256, (kFaceBlockMin<P, PLANAR, SECOND>))
       C br[kBface], wc[5], gc[15], pc[5];
       load_words<P, true>(d.bface + static_cast<long long>(bf) * kBface, 0, kBface, br);
       if (!cell_active(d, index_of(br[13]))) continue;
-      cell_recon<P, SECOND>(d, index_of(br[13]) + z, wc, pc, gc);
+      cell_recon<P, SECOND, true>(d, index_of(br[13]), wc, pc, gc);
       boundary_flux<P, FLUX, PLANAR>(d, bf, br, wc, gc, pc, out);
     }
 #pragma unroll

@@ -2938,6 +2938,7 @@ class Impl final : public Stepper {
     // gradients or limiter; unlimited, phi is 1 (written by the gradient kernel).
     second_ = on;
     ready_plans();
+    repack_blocks();  // the gradients' list of active blocks is kept only while they run
     drop_graph();
   }
 
@@ -3562,8 +3563,10 @@ class Impl final : public Stepper {
   }
 
   // Re-packed launches of batched cases: the blocks of the tuning's plans that hold a cell of a
-  // case still stepping.
+  // case still stepping (the other plans' launches go over all blocks).
   void repack_blocks() {
+    for (GradPlan& p : grad_plans_) p.n_active = -1;
+    for (FacePlan& p : face_plans_) p.n_active = -1;
     auto blocks_of = [&](int nb, Buffer& buf, int& count) {
       count = -1;
       if (n_cell_tiles_ < 0 || active_h_.empty()) return;

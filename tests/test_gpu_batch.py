@@ -107,6 +107,33 @@ def test_every_case_stopped_leaves_the_state_and_the_handle_usable(blocks, graph
         assert bits_equal(a, w)
 
 
+def test_active_cases_changed_while_first_order():
+    """The active cases changed between a second-order step and the next one, while the handle was
+    first order: the gradients run over the blocks of the cases active now, not of those active then."""
+    b = small_batch()
+
+    def run(detour):
+        with device_of(b) as dev:
+            dev.set_active([1, 0, 1])
+            if detour:
+                dev.step(cfl=b.cfl, rk=3, n_steps=1, local=True)
+                dev.set_second_order(False)
+                dev.set_active([0, 1, 0])
+                dev.set_second_order(True)
+                dev.upload(b.u0)
+            else:
+                dev.set_active([0, 1, 0])
+            dev.step(cfl=b.cfl, rk=3, n_steps=3, local=True)
+            return dev.download()
+
+    assert bits_equal(run(True), run(False))
+    o, u1 = case_oracle(b, 1)
+    for _ in range(3):
+        o.step(u1, rk=3, cfl=b.cfl, local=True)
+    c0, c1 = b.cell_offsets[1], b.cell_offsets[2]
+    assert bits_equal(run(True)[:, c0:c1], u1)
+
+
 def test_batched_march_converges_each_case_at_its_own_iteration():
     b = small_batch(cells=(300, 1500), n=4, seed=5)
     with device_of(b) as dev:

@@ -2366,6 +2366,11 @@ struct Failure : std::runtime_error {
   using std::runtime_error::runtime_error;
 };
 
+// No device memory for an allocation.
+struct NoMemory : Failure {
+  using Failure::Failure;
+};
+
 [[noreturn]] void fail(const std::string& what) { throw Failure(what); }
 
 // A failed CUDA call: the runtime's (non-sticky) last-error state is cleared before reporting, so
@@ -2399,7 +2404,16 @@ class Buffer {
     if (p_ != nullptr) cudaFree(p_);
     p_ = nullptr;
     n_ = bytes;
-    if (bytes > 0) check(cudaMalloc(&p_, bytes), "cudaMalloc");
+    if (bytes > 0) {
+      const cudaError_t e = cudaMalloc(&p_, bytes);
+      if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        p_ = nullptr;
+        n_ = 0;
+        throw NoMemory(std::string("E1200: cudaMalloc: ") + cudaGetErrorString(e));
+      }
+      check(e, "cudaMalloc");
+    }
   }
   template <class T>
   T* as() const {
@@ -2864,6 +2878,7 @@ class Impl final : public Stepper {
     check(cudaEventCreateWithFlags(&joined_, cudaEventDisableTiming), "event");
     choose_defaults();
     ready_plans();
+    trim_plans();
     check(cudaStreamSynchronize(stream), "create");
   }
 
@@ -3163,9 +3178,10 @@ class Impl final : public Stepper {
   void set_tuning(const Tuning& t) override {
     t.validate();
     tuning_ = t;
-    ready_plans();
-    repack_blocks();
     drop_graph();
+    ready_plans();
+    trim_plans();
+    repack_blocks();
   }
 
   Tuning tuning() const override { return tuning_; }
@@ -3191,6 +3207,7 @@ class Impl final : public Stepper {
     ensure_flux_scratch();
     auto measure = [&](const Tuning& t, int kind) {
       tuning_ = t;
+      ready_plans();
       double ms[6];
       long long l[6];
       kernel_times(cfl, dt, local, rk, 1, ms, l);
@@ -3203,7 +3220,7 @@ class Impl final : public Stepper {
     };
     Tuning best = tuning_;
     const TrialScope scope = trial_scope(
-        second_, n_, [&](bool mine) { return any_rank(mine); },
+        second_, n_, kFaceBlockCells, [&](bool mine) { return any_rank(mine); },
         [&](int block) { return grad_plan(block) != nullptr; },
         [&](int block) { return face_plan(block) != nullptr; });
     if (second_) {
@@ -3242,6 +3259,7 @@ class Impl final : public Stepper {
     auto step_ms = [&](const Tuning& t) {
       tuning_ = t;
       drop_graph();
+      ready_plans();
       autan_euler_step_result r{};
       cudaEvent_t e0 = nullptr, e1 = nullptr;
       check(cudaEventCreate(&e0), "event");
@@ -3266,7 +3284,6 @@ class Impl final : public Stepper {
     tuning_ = Tuning{};
     choose_defaults();
     const Tuning usual = tuning_;
-    ready_plans();
     double total = step_ms(best);
     const double other = step_ms(usual);
     if (other < total) {
@@ -3274,9 +3291,10 @@ class Impl final : public Stepper {
       best = usual;
     }
     tuning_ = best;
-    ready_plans();
-    repack_blocks();
     drop_graph();
+    ready_plans();
+    trim_plans();
+    repack_blocks();
     return total;
   }
 
@@ -3329,61 +3347,6 @@ class Impl final : public Stepper {
     int n_active = -1;   // re-packed launches: blocks to launch over (-1: all)
   };
 
-  // The gradient plan of `nb` cells per block, built on first use (never inside a capture); null
-  // where a block's neighbourhood does not fit: more candidates than the sort's shared memory
-  // holds, places beyond 16 bits or records beyond the launch's shared memory.
-  GradPlan* grad_plan(int nb) {
-    GradPlan& p = grad_plans_[nb / 32];
-    if (p.built) return p.fits ? &p : nullptr;
-    p.built = true;
-    const int nblk = blocks(n_, nb);
-    long long most = 1;
-    for (int s0 = 0; s0 < nblk; ++s0) {
-      long long sum = 0;
-      for (int c = s0 * nb; c < std::min<long long>(n_, (s0 + 1LL) * nb); ++c) sum += st_.len[c] + inc_.len[c];
-      most = std::max(most, sum);
-    }
-    int cap = 1;
-    while (cap < most && cap < (1 << 20)) cap <<= 1;
-    if (cap > kSortCap) return nullptr;
-    Buffer counts(static_cast<size_t>(nblk) * sizeof(int));
-    const size_t sm = 2ULL * cap * sizeof(int);
-    launch_smem(kControl, k_grad_blocks<P, false>, nblk, nb, sm, d_, cap, counts.as<int>(),
-                static_cast<const int*>(nullptr), static_cast<int*>(nullptr), static_cast<C*>(nullptr),
-                static_cast<C*>(nullptr));
-    std::vector<int> n(nblk), off(nblk + 1, 0);
-    check(cudaMemcpyAsync(n.data(), counts.ptr(), counts.bytes(), cudaMemcpyDeviceToHost, stream), "blocks");
-    check(cudaStreamSynchronize(stream), "blocks");
-    long long run = 0;
-    int largest = 0;
-    for (int i = 0; i < nblk; ++i) {
-      off[i] = static_cast<int>(run);
-      run += n[i];
-      largest = std::max(largest, n[i]);
-      if (run >= std::numeric_limits<int>::max()) return nullptr;
-    }
-    off[nblk] = static_cast<int>(run);
-    GradShape shape{0, 0, nb + largest, 0};
-    const int ns = slices(), per = nb / kSlice;
-    for (int a = 0; a < ns; a += per) {
-      const int e = std::min(a + per, ns);
-      shape.st_rows = std::max(shape.st_rows, st_.start[e] - st_.start[a]);
-      shape.inc_rows = std::max(shape.inc_rows, inc_.start[e] - inc_.start[a]);
-    }
-    for (int c = 0; c < n_; ++c) shape.faces = std::max(shape.faces, inc_.len[c]);
-    if (grad_split_bytes<C>(shape, nb) > kBlockSmem) return nullptr;
-    p.off = upload(off, stream);
-    p.list.alloc(std::max<size_t>(1, static_cast<size_t>(run)) * sizeof(int));
-    p.st.alloc(st_e_.bytes());
-    p.inc.alloc(inc_rec_.bytes());
-    launch_smem(kControl, k_grad_blocks<P, true>, nblk, nb, sm, d_, cap, static_cast<int*>(nullptr),
-                static_cast<const int*>(p.off.template as<int>()), p.list.template as<int>(),
-                p.st.template as<C>(), p.inc.template as<C>());
-    check(cudaStreamSynchronize(stream), "blocks");
-    p.shape = shape;
-    p.fits = true;
-    return &p;
-  }
   struct FacePlan {
     bool built = false, fits = false;
     Buffer first, bfirst, rec, face, bface, inc, inc_start, wfirst, walls, active;
@@ -3399,18 +3362,111 @@ class Impl final : public Stepper {
     }
   };
 
+  // A plan, built by `build` (whether its blocks fit) unless it is; null where they do not fit, for want
+  // of device memory too: the other forms need none of it.
+  template <class Plan, class Build>
+  Plan* built_plan(Plan& p, Build&& build) {
+    if (!p.built) {
+      p.built = true;
+      try {
+        p.fits = build();
+      } catch (const NoMemory&) {
+        p.fits = false;
+      }
+      if (!p.fits) {
+        p = Plan{};
+        p.built = true;
+      }
+    }
+    return p.fits ? &p : nullptr;
+  }
+  GradPlan* grad_plan(int nb) {
+    GradPlan& p = grad_plans_[nb / 32];
+    return built_plan(p, [&] { return build_grad_plan(p, nb); });
+  }
+  FacePlan* face_plan(int nb) {
+    FacePlan& p = face_plans_[nb / 32];
+    return built_plan(p, [&] { return build_face_plan(p, nb); });
+  }
+
+  // The gradient plan of `nb` cells per block (never inside a capture); false where a block's
+  // neighbourhood does not fit: more candidates than the sort's shared memory holds, or rows and
+  // records beyond the launch's shared memory.
+  bool build_grad_plan(GradPlan& p, int nb) {
+    const int nblk = blocks(n_, nb);
+    long long most = 1;
+    for (int s0 = 0; s0 < nblk; ++s0) {
+      long long sum = 0;
+      for (int c = s0 * nb; c < std::min<long long>(n_, (s0 + 1LL) * nb); ++c) sum += st_.len[c] + inc_.len[c];
+      most = std::max(most, sum);
+    }
+    int cap = 1;
+    while (cap < most && cap < (1 << 20)) cap <<= 1;
+    if (cap > kSortCap) return false;
+    Buffer counts(static_cast<size_t>(nblk) * sizeof(int));
+    const size_t sm = 2ULL * cap * sizeof(int);
+    launch_smem(kControl, k_grad_blocks<P, false>, nblk, nb, sm, d_, cap, counts.as<int>(),
+                static_cast<const int*>(nullptr), static_cast<int*>(nullptr), static_cast<C*>(nullptr),
+                static_cast<C*>(nullptr));
+    std::vector<int> n(nblk), off(nblk + 1, 0);
+    check(cudaMemcpyAsync(n.data(), counts.ptr(), counts.bytes(), cudaMemcpyDeviceToHost, stream), "blocks");
+    check(cudaStreamSynchronize(stream), "blocks");
+    long long run = 0;
+    int largest = 0;
+    for (int i = 0; i < nblk; ++i) {
+      off[i] = static_cast<int>(run);
+      run += n[i];
+      largest = std::max(largest, n[i]);
+      if (run >= std::numeric_limits<int>::max()) return false;
+    }
+    off[nblk] = static_cast<int>(run);
+    GradShape shape{0, 0, nb + largest, 0};
+    const int ns = slices(), per = nb / kSlice;
+    for (int a = 0; a < ns; a += per) {
+      const int e = std::min(a + per, ns);
+      shape.st_rows = std::max(shape.st_rows, st_.start[e] - st_.start[a]);
+      shape.inc_rows = std::max(shape.inc_rows, inc_.start[e] - inc_.start[a]);
+    }
+    for (int c = 0; c < n_; ++c) shape.faces = std::max(shape.faces, inc_.len[c]);
+    if (grad_split_bytes<C>(shape, nb) > kBlockSmem) return false;
+    p.off = upload(off, stream);
+    p.list.alloc(std::max<size_t>(1, static_cast<size_t>(run)) * sizeof(int));
+    p.st.alloc(st_e_.bytes());
+    p.inc.alloc(inc_rec_.bytes());
+    launch_smem(kControl, k_grad_blocks<P, true>, nblk, nb, sm, d_, cap, static_cast<int*>(nullptr),
+                static_cast<const int*>(p.off.template as<int>()), p.list.template as<int>(),
+                p.st.template as<C>(), p.inc.template as<C>());
+    check(cudaStreamSynchronize(stream), "blocks");
+    p.shape = shape;
+    return true;
+  }
   // The plans that the tuning's launches take (null where it takes none, or the mesh fits none: the
   // gradients then take the thread-per-cell form, the faces the store-gather one).
   GradPlan* split_plan() {
     if (tuning_.grad_mode != 6 || !second_ || !has_stencil_) return nullptr;
-    return grad_plan(std::min(tuning_.grad_block, kSplitCells));
+    GradPlan& p = grad_plans_[std::min(tuning_.grad_block, kSplitCells) / 32];
+    return p.fits ? &p : nullptr;
   }
-  FacePlan* block_faces() { return tuning_.face_mode == 3 ? face_plan(tuning_.face_block) : nullptr; }
+  FacePlan* block_faces() {
+    if (tuning_.face_mode != 3) return nullptr;
+    FacePlan& p = face_plans_[tuning_.face_block / 32];
+    return p.fits ? &p : nullptr;
+  }
   // Builds what the tuning's launches need (never inside a graph capture).
   void ready_plans() {
-    split_plan();
-    const bool in_blocks = block_faces() != nullptr;
-    if (tuning_.face_mode != 0 && !in_blocks) ensure_flux_scratch();
+    if (tuning_.grad_mode == 6 && second_ && has_stencil_) grad_plan(std::min(tuning_.grad_block, kSplitCells));
+    if (tuning_.face_mode == 3) face_plan(tuning_.face_block);
+    if (tuning_.face_mode != 0 && block_faces() == nullptr) ensure_flux_scratch();
+  }
+  // Frees the plans that the tuning's launches do not take: each is a second copy of the rows or of the
+  // face records.
+  void trim_plans() {
+    const GradPlan* g = split_plan();
+    const FacePlan* f = block_faces();
+    for (GradPlan& p : grad_plans_)
+      if (&p != g) p = GradPlan{};
+    for (FacePlan& p : face_plans_)
+      if (&p != f) p = FacePlan{};
   }
   static constexpr int kSortCap = 16384;
   static constexpr size_t kBlockSmem = 200 * 1024;
@@ -3419,12 +3475,9 @@ class Impl final : public Stepper {
     return 5ULL * static_cast<size_t>(std::max(p.faces, nb)) * sizeof(C);
   }
 
-  // The face plan of `nb` cells per block, built on first use (never inside a capture); null where a
-  // block's faces do not fit (places beyond 15 bits, the sort's or the launch's shared memory).
-  FacePlan* face_plan(int nb) {
-    FacePlan& p = face_plans_[nb / 32];
-    if (p.built) return p.fits ? &p : nullptr;
-    p.built = true;
+  // The face plan of `nb` cells per block (never inside a capture); false where a block's faces do not
+  // fit (places beyond 15 bits, the sort's or the launch's shared memory).
+  bool build_face_plan(FacePlan& p, int nb) {
     const int nblk = blocks(n_, nb);
     long long most = 1;
     for (int b = 0; b < nblk; ++b) {
@@ -3435,7 +3488,7 @@ class Impl final : public Stepper {
     }
     int cap = 1;
     while (cap < most && cap < (1 << 20)) cap <<= 1;
-    if (cap > kSortCap) return nullptr;
+    if (cap > kSortCap) return false;
     Buffer counts(2ULL * nblk * sizeof(int));
     const size_t sm = 2ULL * cap * sizeof(int);
     launch_smem(kControl, k_face_blocks<P, false>, nblk, nb, sm, d_, cap, counts.as<int>(),
@@ -3452,11 +3505,11 @@ class Impl final : public Stepper {
       run += n[2 * b];
       brun += n[2 * b + 1];
       p.faces = std::max(p.faces, n[2 * b] + n[2 * b + 1]);
-      if (run >= std::numeric_limits<int>::max() || brun >= std::numeric_limits<int>::max()) return nullptr;
+      if (run >= std::numeric_limits<int>::max() || brun >= std::numeric_limits<int>::max()) return false;
     }
     first[nblk] = static_cast<int>(run);
     bfirst[nblk] = static_cast<int>(brun);
-    if (p.faces > 32767 || face_block_smem(p, nb) > kBlockSmem) return nullptr;
+    if (p.faces > 32767 || face_block_smem(p, nb) > kBlockSmem) return false;
     std::vector<int> start(inc_.start.size());
     long long rows = 0;
     for (size_t s = 0; s + 1 < inc_.start.size(); ++s) {
@@ -3503,8 +3556,7 @@ class Impl final : public Stepper {
     p.wfirst = upload(wfirst, stream);
     p.walls = upload(walls, stream);
     check(cudaStreamSynchronize(stream), "blocks");
-    p.fits = true;
-    return &p;
+    return true;
   }
 
   // Whether the step's face launches also write the next boundary states.
@@ -3533,6 +3585,7 @@ class Impl final : public Stepper {
   //   computed twice); fp64 tets 38 880 cells 87 / 95, 72 000 cells 166 / 152. Cells and threads a
   //   block: 256 threads to 32 cells at 8 192 cells (38; 128 threads 43), to 64 at 31 154 (68; 32 to
   //   128: 70), 128 to 64 at 60 100 (99; 128 to 128: 110), 128 to 128 at 134 175 (199; 128 to 64: 207).
+  static constexpr long long kFaceBlockCells = 148LL * (sizeof(C) == 4 ? 4096 : 384);
   void choose_defaults() {
     const bool f32 = sizeof(C) == 4;
     const long long per_sm = (static_cast<long long>(n_) + 147) / 148;  // cells
@@ -3541,7 +3594,7 @@ class Impl final : public Stepper {
     else if (f32 && per_sm <= 256) nb = 64, threads = 256;
     else if (!f32 && per_sm <= 128) nb = 32;
     else if (f32 && per_sm <= 512) nb = 64;
-    const FacePlan* f = per_sm <= (f32 ? 4096 : 384) ? face_plan(nb) : nullptr;
+    const FacePlan* f = n_ <= kFaceBlockCells ? face_plan(nb) : nullptr;
     // cell orders whose blocks are not compact (lines or layers of cells) share too many faces between
     // blocks: beyond small meshes, where launches count, no more than 1.4 computations a face
     if (f != nullptr && per_sm > 512 && f->interior > 1.4 * nif_) f = nullptr;

@@ -19,18 +19,21 @@ struct TrialScope {
   bool faces[3] = {false, false, false};
 };
 
-// `any` (bool -> bool): whether any rank has the flag set; every rank calls it together. `split_fits`,
+// `face_cells`: the most cells whose face blocks can win (beyond, their copy of the face records is not
+// made to be tried). `any` (bool -> bool): whether any rank has the flag set; every rank calls it together. `split_fits`,
 // `face_fits` (cells a block -> bool): whether this rank's blocks of that many cells fit.
 template <class Any, class SplitFits, class FaceFits>
-TrialScope trial_scope(bool second, long long cells, Any&& any, SplitFits&& split_fits, FaceFits&& face_fits) {
+TrialScope trial_scope(bool second, long long cells, long long face_cells, Any&& any, SplitFits&& split_fits,
+                       FaceFits&& face_fits) {
   auto all = [&](bool mine) { return !any(!mine); };
   TrialScope s;
   // the split form where every mesh is small enough for it to win
   if (second && all(cells <= 148 * 2048))
     for (int i = 0; i < 2; ++i) s.split[i] = all(split_fits(kSplitTrials[i]));
   s.small = all(cells <= 148 * 512);
+  const bool blocks = all(cells <= face_cells);
   for (int i = 0; i < 3; ++i)
-    if (s.small || kFaceTrials[i] == 128) s.faces[i] = all(face_fits(kFaceTrials[i]));
+    if (s.small || (blocks && kFaceTrials[i] == 128)) s.faces[i] = all(face_fits(kFaceTrials[i]));
   return s;
 }
 

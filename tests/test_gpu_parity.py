@@ -315,6 +315,60 @@ def test_block_forms_are_bit_identical(build, precision):
             assert bits_equal(a, b), (tuning, graph, between)
 
 
+def test_a_handle_keeps_only_the_plans_its_launches_take():
+    """The blocks of cells that tuning tried and left are freed: a tuned handle holds the memory of one
+    that was given its choices; changing them gives back what the new ones do not take."""
+    case = cases.vortex_tets(16, 16, 6, precision="fp32+acc64")
+    with EulerDevice(case.mesh, case.scheme, case.bc_kind, case.bc_data) as dev:
+        dev.upload(case.u0)
+        dev.set_tuning(grad_mode=0, grad_chunk=2, grad_block=64, face_mode=1, face_block=64, gather_block=128)
+        plain = dev.counters()["device_bytes"]  # with the face scratch, without blocks
+        tuned, _ = dev.autotune(cfl=case.cfl, rk=3, trial_steps=1)
+        after = dev.counters()["device_bytes"]
+        dev.set_tuning(grad_mode=0, grad_chunk=2, grad_block=64, face_mode=1, face_block=64, gather_block=128)
+        assert dev.counters()["device_bytes"] == plain
+        dev.set_tuning(**tuned)
+        assert dev.counters()["device_bytes"] == after
+
+
+def test_blocks_that_find_no_device_memory_leave_the_other_forms():
+    """With the device's memory taken, the block forms' plans cannot be had: the handle's choice of them
+    runs the store-gather and thread-per-cell forms, tuning does without them, same bits."""
+    import torch
+
+    case = cases.bump_channel(96, 75, 75, steps=2)
+    with EulerDevice(case.mesh, case.scheme, case.bc_kind, case.bc_data) as dev:
+        plain = dict(grad_mode=0, grad_chunk=2, grad_block=64, face_mode=1, face_block=64, gather_block=128)
+
+        def march(tuning):
+            dev.set_tuning(**tuning)
+            dev.upload(case.u0)
+            r = dev.step(cfl=case.cfl, local=case.local, rk=case.rk, n_steps=2)
+            return dev.download(), np.array(r.residuals)
+
+        want = march(plain)
+        held, size = [], 1 << 34
+        dev.autotune(cfl=case.cfl, local=case.local, rk=case.rk, trial_steps=1)  # the kernels loaded
+        march(plain)
+        before = dev.counters()["device_bytes"]
+        try:
+            while size >= 1 << 24:  # all but about 100 MB
+                free, _ = torch.cuda.mem_get_info()
+                if free - size < 100 << 20:
+                    size >>= 1
+                    continue
+                held.append(torch.empty(size, dtype=torch.uint8, device="cuda:0"))
+            got = march(dict(plain, face_mode=3, face_block=128, gather_block=128, grad_mode=6, grad_block=32))
+            assert dev.counters()["device_bytes"] == before
+            tuned, _ = dev.autotune(cfl=case.cfl, local=case.local, rk=case.rk, trial_steps=1)
+        finally:
+            held.clear()
+            torch.cuda.empty_cache()
+        for a, b in zip(got, want):
+            assert bits_equal(a, b)
+        assert tuned["face_mode"] != 3 and tuned["grad_mode"] != 6
+
+
 @pytest.mark.parametrize("n", [(17, 15, 3), (400, 340, 1), (1060, 1000, 1)], ids=["765", "136k", "1060k"])
 def test_states_come_back_as_they_went(n):
     """A state to the device and back three times from pageable memory: rows through the handle's pinned

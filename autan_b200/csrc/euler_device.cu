@@ -2888,7 +2888,6 @@ class Impl final : public Stepper {
   }
   void release() {
     if (head_ != nullptr) cudaFreeHost(head_);
-    if (rows_host_ != nullptr) cudaFreeHost(rows_host_);
     if (side_ != nullptr) cudaStreamDestroy(side_);
     if (forked_ != nullptr) cudaEventDestroy(forked_);
     if (joined_ != nullptr) cudaEventDestroy(joined_);
@@ -2988,24 +2987,21 @@ class Impl final : public Stepper {
   }
   void copy_out(const double* dev, double* host, bool zero_images = false) {
     const size_t per = static_cast<size_t>(n_) * sizeof(double);
-    if (HostStage::pinned(host)) {
+    const bool pinned = HostStage::pinned(host);
+    // a small state into pinned memory of the handle's in one copy, then the rows (31 000 cells: 109 us;
+    // one 2-D copy into the caller's 271, a copy a component 336). It takes a millisecond or two to get:
+    // not for a handle's first copies
+    char* rows = nullptr;
+    if (!pinned && per < kRowsPinned && (rows_host_.held() || ++copies_out_ > 2))
+      rows = static_cast<char*>(rows_host_.get(5 * per));
+    if (rows != nullptr) {
+      check(cudaMemcpyAsync(rows, dev, 5 * per, cudaMemcpyDeviceToHost, stream), "download");
+      check(cudaStreamSynchronize(stream), "download");
+      for (int k = 0; k < 5; ++k) std::memcpy(host + k * static_cast<long long>(nc_), rows + k * per, per);
+    } else if (pinned || per < kRowsAtOnce) {
       check(cudaMemcpy2DAsync(host, static_cast<size_t>(nc_) * sizeof(double), dev, per, per, 5,
                               cudaMemcpyDeviceToHost, stream), "download");
       check(cudaStreamSynchronize(stream), "download");
-    } else if (per < kRowsAtOnce && (per >= kRowsPinned || (++copies_out_ <= 2 && rows_host_ == nullptr))) {
-      // (pinned memory takes a millisecond or two to get: not for a handle's first copies)
-      check(cudaMemcpy2DAsync(host, static_cast<size_t>(nc_) * sizeof(double), dev, per, per, 5,
-                              cudaMemcpyDeviceToHost, stream), "download");
-      check(cudaStreamSynchronize(stream), "download");
-    } else if (per < kRowsAtOnce) {
-      // one copy into pinned memory of the handle's, then the rows (31 000 cells: 109 us; one 2-D copy
-      // into the caller's 271, a copy a component 336)
-      if (rows_host_ == nullptr)
-        check(cudaMallocHost(reinterpret_cast<void**>(&rows_host_), 5 * per), "cudaMallocHost");
-      check(cudaMemcpyAsync(rows_host_, dev, 5 * per, cudaMemcpyDeviceToHost, stream), "download");
-      check(cudaStreamSynchronize(stream), "download");
-      for (int k = 0; k < 5; ++k)
-        std::memcpy(host + k * static_cast<long long>(nc_), rows_host_ + k * static_cast<long long>(n_), per);
     } else {
       if (!out_stage_) out_stage_ = HostStage::of_device(1);
       ++copies_out_;
@@ -4523,7 +4519,7 @@ class Impl final : public Stepper {
   bool chained_ = false;  // set around launches of kernels that wait for the previous one themselves
   bool step_tiles_ = false;  // set while enqueue_step records: its launches use the tiles
   Control* head_ = nullptr;  // pinned copy of the control's head
-  double* rows_host_ = nullptr;  // pinned rows of a small state on its way out
+  HostRows rows_host_;  // pinned rows of a small state on its way out
   std::shared_ptr<HostStage> in_stage_, out_stage_;
   int copies_in_ = 0, copies_out_ = 0;  // the handle's pageable state copies so far
   cudaStream_t side_ = nullptr;  // a step's norms, beside its later stages

@@ -181,4 +181,29 @@ class HostStage {
   Slot slots_[2 * kLanes];
 };
 
+// Pinned memory of one handle's, got on first use; where none is to be had it stays without.
+class HostRows {
+ public:
+  HostRows() = default;
+  HostRows(const HostRows&) = delete;
+  HostRows& operator=(const HostRows&) = delete;
+  ~HostRows() {
+    if (p_ != nullptr) cudaFreeHost(p_);
+  }
+  bool held() const { return p_ != nullptr; }
+  // `bytes` (the same at every call) of it, or null.
+  void* get(size_t bytes) {
+    if (p_ == nullptr && !refused_ && cudaMallocHost(&p_, bytes) != cudaSuccess) {
+      (void)cudaGetLastError();
+      p_ = nullptr;
+      refused_ = true;
+    }
+    return p_;
+  }
+
+ private:
+  void* p_ = nullptr;
+  bool refused_ = false;
+};
+
 }  // namespace autan_b200

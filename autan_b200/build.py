@@ -44,7 +44,8 @@ HOST_SOURCES = ["setup.cpp"]
 CUDA_SOURCES = ["euler_device.cu", "norms_static.cu", "mlp.cu", "setup_device.cu"]
 HEADERS = ["euler_bodies.cuh", "exact_sum.cuh", "device_mesh.hpp", "convergence.hpp",
            "setup_rules.cuh", "mlp_fused.cuh", "cell_blocks.cuh",
-           "face_blocks.cuh", "host_stage.hpp", "tuning_trials.hpp"]
+           "face_blocks.cuh", "host_stage.hpp", "tuning_trials.hpp",
+           "piece_ring.hpp"]
 
 
 def _newer(src: Path, obj: Path, deps: list[Path]) -> bool:

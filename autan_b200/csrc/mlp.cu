@@ -17,7 +17,6 @@
 #include <stdio.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -28,6 +27,7 @@
 
 #include "autan_mlp.h"
 #include "host_stage.hpp"
+#include "piece_ring.hpp"
 
 namespace autan_b200 {
 namespace mlp {
@@ -1156,49 +1156,24 @@ class Net {
     }
     const long long pieces = (n + kPredictPiece - 1) / kPredictPiece;
     auto rows_of = [&](long long p) { return static_cast<int>(std::min(kPredictPiece, n - p * kPredictPiece)); };
-    std::atomic<long long> launched{0}, drained{0};
-    std::atomic<bool> stop{false};
-    std::exception_ptr failed;
     get_stage();
-    auto drain = [&] {
-      try {
-        check(cudaSetDevice(device_), "cudaSetDevice");
-        for (long long p = 0; p < pieces; ++p) {
-          while (launched.load(std::memory_order_acquire) <= p) {
-            if (stop.load()) return;
-            std::this_thread::yield();
-          }
+    run_pieces(
+        pieces, kRing,
+        [&](long long p) {
           const int b = static_cast<int>(p % kRing);
+          float* xs = px_.as<float>() + b * xp;
+          put(xs, x + p * kPredictPiece * inputs_, static_cast<size_t>(rows_of(p)) * inputs_ * 4);
+          predict_rows(xs, rows_of(p), py_.as<float>() + b * yp);
+          check(cudaEventRecord(ring_done_[b], stream_), "predict");
+        },
+        [&](long long p) {
+          const int b = static_cast<int>(p % kRing);
+          if (p == 0) check(cudaSetDevice(device_), "cudaSetDevice");
           check(cudaStreamWaitEvent(out_stream_, ring_done_[b], 0), "predict");
           get(y + p * kPredictPiece * outputs_, py_.as<float>() + b * yp,
               static_cast<size_t>(rows_of(p)) * outputs_ * 4, out_stream_);
           check(cudaStreamSynchronize(out_stream_), "predict");  // (the caller's memory may be pinned)
-          drained.store(p + 1, std::memory_order_release);
-        }
-      } catch (...) {
-        failed = std::current_exception();
-        stop.store(true);
-      }
-    };
-    std::thread out(drain);
-    try {
-      for (long long p = 0; p < pieces && !stop.load(); ++p) {
-        while (p - drained.load(std::memory_order_acquire) >= kRing && !stop.load()) std::this_thread::yield();
-        if (stop.load()) break;
-        const int b = static_cast<int>(p % kRing);
-        float* xs = px_.as<float>() + b * xp;
-        put(xs, x + p * kPredictPiece * inputs_, static_cast<size_t>(rows_of(p)) * inputs_ * 4);
-        predict_rows(xs, rows_of(p), py_.as<float>() + b * yp);
-        check(cudaEventRecord(ring_done_[b], stream_), "predict");
-        launched.store(p + 1, std::memory_order_release);
-      }
-    } catch (...) {
-      stop.store(true);
-      out.join();
-      throw;
-    }
-    out.join();
-    if (failed) std::rethrow_exception(failed);
+        });
   }
 
   // One forward and backward pass on host rows, no update: the loss and the gradient.

@@ -142,18 +142,33 @@ def test_engines_agree(rows):
 
 @pytest.mark.parametrize("engine", [0, 2])
 def test_prediction_in_pieces(engine):
-    """More rows than one piece (2^17) and than the ring of pieces holds, a ragged last one: the rows of
-    one call equal those of calls of their own, whatever they share a piece with."""
+    """More rows than one piece (2^17) and than the ring of pieces holds, a ragged last one: every row
+    equals its prediction in a small call of its own (below the pinned slots' least size), on a handle's
+    first call (the driver's copies), on its later ones (both directions through the slots, on two
+    threads) with other rows each, and between pinned arrays."""
+    import ctypes as C
+
+    import torch
+
     n = 4 * 131072 + 77
     x, y = data(20000, seed=13)
     x = np.concatenate([x] * (n // 20000 + 1))[:n]
-    x[::3] *= 0.5
     net = MLP(seed=14)
     net.set_engine(engine)
     net.set_scaling(*scaling(x[:20000], y))
-    got = net.predict(x)
-    for a, b in ((0, 1000), (131072 - 300, 131072 + 300), (400000, 400128), (n - 77, n)):
-        assert np.array_equal(got[a:b], net.predict(x[a:b]))
+    rng = np.random.default_rng(15)
+    for call in range(4):
+        xc = x * rng.uniform(0.5, 1.0, (n, 1)).astype(np.float32)
+        if call < 3:
+            got = net.predict(xc)
+        else:
+            xp = torch.from_numpy(xc).pin_memory()
+            yp = torch.zeros((n, got.shape[1]), dtype=torch.float32).pin_memory()
+            f32 = C.POINTER(C.c_float)
+            net._call("autan_mlp_predict", C.cast(xp.data_ptr(), f32), n, C.cast(yp.data_ptr(), f32), 0)
+            got = yp.numpy()
+        want = np.concatenate([net.predict(xc[a : a + 20000]) for a in range(0, n, 20000)])
+        assert np.array_equal(got, want), call
 
 
 def test_fused_engine_is_the_default_and_deterministic():

@@ -18,6 +18,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstring>
 #include <memory>
 #include <random>
@@ -1118,6 +1119,13 @@ class Net {
       predict_rows(px_.as<float>(), static_cast<int>(n), py_.as<float>());
       get(y, py_.p, static_cast<size_t>(n) * outputs_ * 4, stream_);
     } else {
+      // predictions leave before later rows are read: rows that share memory with them are put aside
+      std::vector<float> aside;
+      const auto at = [](const float* p) { return reinterpret_cast<uintptr_t>(p); };
+      if (at(x) < at(y + n * outputs_) && at(y) < at(x + n * inputs_)) {
+        aside.assign(x, x + n * inputs_);
+        x = aside.data();
+      }
       predict_pieces(x, n, y);
     }
     sync();

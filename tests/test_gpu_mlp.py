@@ -171,6 +171,25 @@ def test_prediction_in_pieces(engine):
         assert np.array_equal(got, want), call
 
 
+def test_prediction_into_its_own_rows():
+    """Predictions over the memory of the rows they come from, more of them than inputs, in many pieces:
+    as into an array of their own."""
+    import ctypes as C
+
+    n, ins, outs = 8 * 131072 + 5, 3, 9
+    rng = np.random.default_rng(21)
+    net = MLP(inputs=ins, outputs=outs, seed=22)
+    x = rng.standard_normal((n, ins)).astype(np.float32)
+    want = net.predict(x)
+    buf = np.zeros(n * outs, dtype=np.float32)
+    f32 = C.POINTER(C.c_float)
+    for _ in range(2):
+        buf[: n * ins] = x.ravel()
+        p = buf.ctypes.data_as(f32)
+        net._call("autan_mlp_predict", p, n, p, 0)
+        assert np.array_equal(buf.reshape(n, outs), want)
+
+
 def test_fused_engine_is_the_default_and_deterministic():
     """Width 128: the fused engine unless another is chosen; two passes give the same bits (the
     CTAs' partials are summed in a fixed order); other widths refuse it."""

@@ -2548,8 +2548,8 @@ struct Tuning {
 
 void Tuning::validate() const {
   auto block_ok = [](int b) { return b >= 32 && b <= 256 && b % 32 == 0; };
-  if (grad_mode == 0 && grad_chunk != 1 && grad_chunk != 2 && grad_chunk != 4 && grad_chunk != 8)
-    fail("E1101: grad_chunk is 1, 2 or 4 (8: as 4)");
+  if (grad_mode == 0 && grad_chunk != 1 && grad_chunk != 2 && grad_chunk != 4)
+    fail("E1101: grad_chunk is 1, 2 or 4");
   if (grad_mode == 0 && grad_chunk == 2 && grad_block > 128)
     fail("E1101: the gradient kernel with 2 entries in flight takes <= 128 threads");
   if (grad_mode == 1 && grad_chunk != 2 && grad_chunk != 4 && grad_chunk != 8)

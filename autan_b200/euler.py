@@ -344,11 +344,16 @@ class EulerDevice:
         self._call("autan_euler_device_get_tuning", N.ptr(p, C.c_int32), len(p))
         return dict(zip(self.TUNING_KEYS, map(int, p)))
 
+    _mode_chosen = False  # a gradient form set by set_tuning or autotune
+
     def set_tuning(self, **kw) -> None:
         t = self.tuning()
+        if kw.get("grad_chunk") == 8 and "grad_mode" not in kw and not self._mode_chosen:
+            t["grad_mode"] = 1  # of a new handle's choices only the staged form takes eight
         t.update(kw)
         p = np.array([t[k] for k in self.TUNING_KEYS], dtype=np.int32)
         self._call("autan_euler_device_set_tuning", N.ptr(p, C.c_int32), len(p))
+        self._mode_chosen = self._mode_chosen or "grad_mode" in kw
 
     def autotune(self, cfl: float = 0.8, dt: float = 0.0, local: bool = False, rk: int = 3,
                  trial_steps: int = 2) -> tuple[dict, float]:  # fmt: skip
@@ -357,6 +362,7 @@ class EulerDevice:
         ms = C.c_double()
         self._call("autan_euler_device_autotune", float(cfl), float(dt), int(local), int(rk),
                    int(trial_steps), N.ptr(p, C.c_int32), C.byref(ms))  # fmt: skip
+        self._mode_chosen = True
         return dict(zip(self.TUNING_KEYS, map(int, p))), float(ms.value)
 
     def set_stall_test(self, polls: int) -> None:

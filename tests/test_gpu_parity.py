@@ -235,6 +235,23 @@ def test_tuning_variants_are_bit_identical(precision):
         assert bits_equal(rms, rms_o), v
 
 
+def test_eight_entries_in_flight_are_the_staged_forms():
+    """grad_chunk 8 is refused for the form that each thread loads its own rows in, and on a new handle
+    (whatever form it took) is the staged form's."""
+    from autan_b200._native import NativeError
+
+    case = cases.vortex_tets(8, 8, 4)
+    with EulerDevice(case.mesh, case.scheme, case.bc_kind, case.bc_data) as dev:
+        dev.set_tuning(grad_chunk=8)
+        assert (dev.tuning()["grad_mode"], dev.tuning()["grad_chunk"]) == (1, 8)
+        for kw in (dict(grad_mode=0), dict(grad_mode=0, grad_chunk=8)):
+            with pytest.raises(NativeError, match="E1101"):
+                dev.set_tuning(**kw)
+        dev.set_tuning(grad_mode=0, grad_chunk=2)
+        with pytest.raises(NativeError, match="E1101"):
+            dev.set_tuning(grad_chunk=8)
+
+
 @pytest.mark.parametrize("precision", ["fp64", "fp32+acc64"])
 def test_gradient_stagings_agree_on_the_channel(precision):
     """The hybrid bump channel (hexahedra, prisms and polyhedral bricks: about 23 stencil entries

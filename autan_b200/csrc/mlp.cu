@@ -83,27 +83,36 @@ __device__ __forceinline__ void mma16816(float* d, const uint32_t* a, const uint
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// GELU(z) = z Phi(z) and its derivative Phi(z) + z phi(z), the erf form, from one exponential: with
-// u = |z| / sqrt(2), erfc(u) = exp(-u^2) (c1 t + ... + c6 t^6), t = 1 / (1 + 0.39 u), the form of
-// Hastings (Approximations for Digital Computers, 1955) with coefficients fitted here (the largest
-// error of erfc 8e-9 over u >= 0, below FP32's own rounding); exp(-u^2) = exp(-z^2 / 2) also gives phi.
-// Against FP64 over [-9, 9]: GELU 5.7e-8 rms and 3.8e-7 at most, its derivative 2.4e-8 and 1.5e-7 (by
-// erff and expf: 6.4e-8, 4.5e-7, 2.4e-8 and 1.2e-7). About 20 instructions for the pair, where erff
-// and expf together take three times as many, and the fused engine's epilogues are bound by them: its
-// prediction of 2^18 rows went from 250 to 209 us, its training pass of 8 192 rows (with the 32-byte
-// stores of the weight gradients) from 95 to 45 us.
+// GELU(z) = z Phi(z) and its derivative Phi(z) + z phi(z), the erf form, from one exponential
+// e = exp(-z^2 / 2), which also gives phi. Below |z| = 1.2, Phi = 1/2 + z P(z^2), a polynomial fitted
+// here (the largest error of Phi 1.3e-9): Phi rounds once there. Above, where Phi's tail is at most 0.115
+// and its relative error counts a tenth, Phi(-|z|) = e (c1 t + ... + c5 t^5), t = 1 / (1 + 0.2758 |z|),
+// the form of Hastings (Approximations for Digital Computers, 1955) with coefficients fitted here
+// (5.2e-9 at most). Against FP64, 6 million values in [-9, 9]: GELU 4.9e-8 rms and 3.8e-7 at most, its
+// derivative 2.4e-8 and 1.4e-7; by erff and expf 5.7e-8 and 4.9e-7, 2.7e-8 and 1.5e-7. About 28
+// instructions for the pair, where erff and expf together take twice as many, and the fused engine's
+// epilogues are bound by them: its prediction of 2^18 rows takes 229 us, by erff and expf 250 (209 by
+// Hastings' form at every z, whose derivative is off by up to 2.2e-7), its training pass of 8 192 rows
+// (with the 32-byte stores of the weight gradients) 46 us where it took 95.
 __device__ __forceinline__ void gelu_pair(float z, float* y, float* dy) {
+  const float s = z * z;
   float t, e;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(__fmaf_rn(0.275771645f, fabsf(z), 1.0f)));
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z * z * -0.721347520f));
-  float p = -0.227536921f;
-  p = __fmaf_rn(p, t, 0.886663537f);
-  p = __fmaf_rn(p, t, -0.635398924f);
-  p = __fmaf_rn(p, t, 0.649558305f);
-  p = __fmaf_rn(p, t, 0.091388853f);
-  p = __fmaf_rn(p, t, 0.235325149f);
-  const float q = 0.5f * (p * t) * e;
-  const float cdf = z > 0.0f ? 1.0f - q : q;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(__fmaf_rn(0.2758f, fabsf(z), 1.0f)));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(s * -0.721347520f));
+  float p = 0.0607838989f;
+  p = __fmaf_rn(p, t, 0.195468578f);
+  p = __fmaf_rn(p, t, -0.0185639311f);
+  p = __fmaf_rn(p, t, 0.160284720f);
+  p = __fmaf_rn(p, t, 0.102419286f);
+  const float q = (p * t) * e;
+  float r = -6.82739842e-6f;
+  r = __fmaf_rn(r, s, 1.11010820e-4f);
+  r = __fmaf_rn(r, s, -1.18363062e-3f);
+  r = __fmaf_rn(r, s, 9.97203706e-3f);
+  r = __fmaf_rn(r, s, -0.0664901109f);
+  r = __fmaf_rn(r, s, 0.398942267f);
+  const float tail = z > 0.0f ? 1.0f - q : q;
+  const float cdf = fabsf(z) < 1.2f ? __fmaf_rn(z, r, 0.5f) : tail;
   *y = z * cdf;
   *dy = __fmaf_rn(z, e * 0.398942280f, cdf);
 }
@@ -770,6 +779,11 @@ __global__ void __launch_bounds__(128) k_wall_distance(const double* tri, const 
     }
   }
   out[i] = sqrt(best);
+}
+
+__global__ void k_gelu(const float* z, long long n, float* y, float* dy) {
+  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i < n) gelu_pair(z[i], y + i, dy + i);
 }
 
 // ---------------------------------------------------------------- host
@@ -1517,6 +1531,20 @@ int autan_mlp_predict(void* handle, const float* x, int64_t n, float* y, int32_t
     if (x == nullptr || y == nullptr || n < 0) fail("E1101: null arrays");
     if (n == 0) return;
     as_net(handle)->predict(x, n, y, device_ptrs != 0);
+  });
+}
+
+int autan_mlp_gelu(const float* z, int64_t n, float* y, float* dy, char* err, size_t err_len) {
+  return guarded(err, err_len, [&] {
+    if (z == nullptr || y == nullptr || dy == nullptr || n < 1 || n > (int64_t(1) << 31))
+      fail("E1101: 1 to 2^31 values and non-null arrays");
+    const size_t bytes = static_cast<size_t>(n) * 4;
+    Buf zd(bytes), yd(bytes), dd(bytes);
+    check(cudaMemcpy(zd.p, z, bytes, cudaMemcpyHostToDevice), "copy");
+    k_gelu<<<blocks(n, 256), 256>>>(zd.as<float>(), n, yd.as<float>(), dd.as<float>());
+    check(cudaGetLastError(), "gelu");
+    check(cudaMemcpy(y, yd.p, bytes, cudaMemcpyDeviceToHost), "copy");
+    check(cudaMemcpy(dy, dd.p, bytes, cudaMemcpyDeviceToHost), "copy");
   });
 }
 

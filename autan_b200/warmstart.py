@@ -41,6 +41,7 @@ def _bind():
     fn("autan_mlp_set_data", C.c_int, vp, P(f32), P(f32), i64, C.c_char_p, sz)
     fn("autan_mlp_train", C.c_int, vp, i32, i32, f32, u64, P(f32), C.c_char_p, sz)
     fn("autan_mlp_gradient", C.c_int, vp, P(f32), P(f32), i64, P(f32), P(f32), C.c_char_p, sz)
+    fn("autan_mlp_gelu", C.c_int, P(f32), i64, P(f32), P(f32), C.c_char_p, sz)
     fn("autan_mlp_predict", C.c_int, vp, P(f32), i64, P(f32), i32, C.c_char_p, sz)
     fn("autan_wall_distance", C.c_int, P(f64), P(i64), P(f64), P(i64), i32, i64, P(f64),
        C.c_char_p, sz)  # fmt: skip
@@ -151,6 +152,16 @@ def wall_triangles(mesh, zone: int) -> np.ndarray:
         for i in range(len(nodes)):
             out.append(np.concatenate([m, p[i], p[(i + 1) % len(nodes)]]))
     return np.array(out).reshape(-1, 9)
+
+
+def gelu(z) -> tuple:
+    """(GELU(z), its derivative) as the hidden layers' kernels form them (test hook)."""
+    z = _f32(z).ravel()
+    y, dy = np.zeros_like(z), np.zeros_like(z)
+    err = N.errbuf()
+    N.check(_bind().autan_mlp_gelu(N.ptr(z, C.c_float), z.size, N.ptr(y, C.c_float), N.ptr(dy, C.c_float),
+                                   err, len(err)), err)  # fmt: skip
+    return y, dy
 
 
 def wall_distance(triangles: list, points: list) -> list:

@@ -68,6 +68,10 @@ int autan_mlp_gradient(void* handle, const float* x, const float* y, int64_t n, 
 int autan_mlp_predict(void* handle, const float* x, int64_t n, float* y, int32_t device_ptrs,
                       char* err, size_t err_len);
 
+/* Test hook of the hidden layers' activation: y = GELU(z) (the erf form) and dy = its derivative as the
+ * kernels form them, n values; host arrays, on the current device. */
+int autan_mlp_gelu(const float* z, int64_t n, float* y, float* dy, char* err, size_t err_len);
+
 /* Wall distance, exact in FP64 (the point-triangle projection of WallSurface::distance,
  * core/include/autan/core/wall_distance.hpp:28-31): for every point i of case k (points
  * [point_offsets[k], point_offsets[k + 1])), the distance to the nearest of that case's wall

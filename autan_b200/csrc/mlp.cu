@@ -638,7 +638,7 @@ constexpr int kFan = 8;
 constexpr int kTreeLevels = 24;
 struct CaseTree {
   int64_t tri0;        // the case's first triangle
-  int n;               // its triangles
+  int64_t n;           // its triangles
   int levels;          // levels of its tree, level 0 the leaves (0: no triangles)
   int at[kTreeLevels];    // each level's first node
   int count[kTreeLevels];
@@ -682,7 +682,9 @@ __global__ void k_wall_nodes(const double* tri, const CaseTree* trees, int level
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < T.count[level]; i += gridDim.x * blockDim.x) {
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     if (level == 0) {
-      for (int t = i * kLeaf; t < min(T.n, (i + 1) * kLeaf); ++t) widen_by(tri + 9 * (T.tri0 + t), lo, hi);
+      const int64_t t0 = static_cast<int64_t>(i) * kLeaf;
+      const int nt = static_cast<int>(T.n - t0 < kLeaf ? T.n - t0 : kLeaf);
+      for (int t = 0; t < nt; ++t) widen_by(tri + 9 * (T.tri0 + t0 + t), lo, hi);
     } else {
       const int c1 = min(T.count[level - 1], (i + 1) * kFan);
       for (int c = i * kFan; c < c1; ++c) {
@@ -701,12 +703,12 @@ __global__ void k_wall_nodes(const double* tri, const CaseTree* trees, int level
 // 0.69 ms through the tree.
 __global__ void __launch_bounds__(128) k_wall_distance(const double* tri, const CaseTree* trees,
                                                        const float4* nodes, const int64_t* pt_off,
-                                                       int n_cases, const double* pts, long long n,
+                                                       int n_runs, const double* pts, long long n,
                                                        double* out) {
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int k = 0;
-  for (int hi = n_cases - 1; k < hi;) {  // the case whose points hold i
+  for (int hi = n_runs - 1; k < hi;) {  // the run of points that holds i
     const int m = (k + hi + 1) >> 1;
     if (pt_off[m] <= i) k = m;
     else hi = m - 1;
@@ -715,8 +717,10 @@ __global__ void __launch_bounds__(128) k_wall_distance(const double* tri, const 
   const V3 p{pts[i], pts[n + i], pts[2 * n + i]};
   double best = __longlong_as_double(0x7ff0000000000000LL);
   auto leaf = [&](int l) {
-    for (int t = l * kLeaf; t < min(T.n, (l + 1) * kLeaf); ++t) {
-      const double* q = tri + 9 * (T.tri0 + t);
+    const int64_t t0 = static_cast<int64_t>(l) * kLeaf;
+    const int nt = static_cast<int>(T.n - t0 < kLeaf ? T.n - t0 : kLeaf);
+    for (int t = 0; t < nt; ++t) {
+      const double* q = tri + 9 * (T.tri0 + t0 + t);
       const double d = point_triangle2(p, {q[0], q[1], q[2]}, {q[3], q[4], q[5]}, {q[6], q[7], q[8]});
       if (d < best) best = d;
     }
@@ -1565,8 +1569,7 @@ int autan_wall_distance(const double* triangles, const int64_t* tri_offsets, con
       T = CaseTree{};
       T.tri0 = tri_offsets[k];
       const int64_t n = std::max<int64_t>(0, tri_offsets[k + 1] - tri_offsets[k]);
-      if (n > (1LL << 30)) fail("E1101: too many triangles in one case");
-      T.n = static_cast<int>(n);
+      T.n = n;
       for (int64_t c = (n + kLeaf - 1) / kLeaf; c > 0; c = (c + kFan - 1) / kFan) {
         if (n_nodes + c > (1LL << 31) - 1) fail("E1101: too many triangles");
         T.at[T.levels] = static_cast<int>(n_nodes);
@@ -1577,7 +1580,24 @@ int autan_wall_distance(const double* triangles, const int64_t* tri_offsets, con
       }
       levels = std::max(levels, T.levels);
     }
-    // one allocation: triangles, trees, nodes, point offsets, points, distances
+    // runs of points of one case each: the cases' own where they follow one another; where their ranges
+    // overlap a point is the last such case's, outside them all the first's
+    std::vector<int64_t> runs(point_offsets, point_offsets + n_cases);
+    std::vector<CaseTree> run_trees;
+    if (!std::is_sorted(point_offsets, point_offsets + n_cases + 1)) {
+      std::vector<int> case_of(static_cast<size_t>(n_points), 0);
+      for (int k = 0; k < n_cases; ++k)
+        for (int64_t i = std::max<int64_t>(point_offsets[k], 0); i < std::min(point_offsets[k + 1], n_points); ++i)
+          case_of[i] = k;
+      runs.clear();
+      for (int64_t i = 0; i < n_points; ++i)
+        if (i == 0 || case_of[i] != case_of[i - 1]) {
+          runs.push_back(i);
+          run_trees.push_back(trees[case_of[i]]);
+        }
+    }
+    const int n_runs = static_cast<int>(runs.size());
+    // one allocation: triangles, trees, nodes, runs, points, distances
     const size_t np = static_cast<size_t>(std::max<int64_t>(n_points, 1));
     size_t total = 0;
     auto take = [&](size_t bytes) {
@@ -1588,7 +1608,7 @@ int autan_wall_distance(const double* triangles, const int64_t* tri_offsets, con
     const size_t o_tri = take(static_cast<size_t>(std::max<int64_t>(nt, 1)) * 72),
                  o_tree = take(static_cast<size_t>(n_cases) * sizeof(CaseTree)),
                  o_node = take(static_cast<size_t>(std::max<int64_t>(n_nodes, 1)) * 32),
-                 o_off = take((static_cast<size_t>(n_cases) + 1) * 8),
+                 o_off = take(runs.size() * 8), o_run = take(run_trees.size() * sizeof(CaseTree)),
                  o_pts = take(np * 24), o_out = take(np * 8);
     Buf mem(total);
     unsigned char* m = mem.as<unsigned char>();
@@ -1596,11 +1616,14 @@ int autan_wall_distance(const double* triangles, const int64_t* tri_offsets, con
     auto* tree = reinterpret_cast<CaseTree*>(m + o_tree);
     auto* node = reinterpret_cast<float4*>(m + o_node);
     auto* off = reinterpret_cast<int64_t*>(m + o_off);
+    auto* run_tree = run_trees.empty() ? tree : reinterpret_cast<CaseTree*>(m + o_run);
     auto* pts = reinterpret_cast<double*>(m + o_pts);
     auto* out = reinterpret_cast<double*>(m + o_out);
     if (nt > 0) check(cudaMemcpy(tri, triangles, nt * 9 * 8, cudaMemcpyHostToDevice), "copy");
     check(cudaMemcpy(tree, trees.data(), trees.size() * sizeof(CaseTree), cudaMemcpyHostToDevice), "copy");
-    check(cudaMemcpy(off, point_offsets, (n_cases + 1) * 8, cudaMemcpyHostToDevice), "copy");
+    check(cudaMemcpy(off, runs.data(), runs.size() * 8, cudaMemcpyHostToDevice), "copy");
+    if (!run_trees.empty())
+      check(cudaMemcpy(run_tree, run_trees.data(), run_trees.size() * sizeof(CaseTree), cudaMemcpyHostToDevice), "copy");
     // (the pinned slots are worth their allocation from some tens of megabytes; there is no handle here
     // that would keep them from one call to the next)
     const bool staged = n_points > (1 << 21);
@@ -1616,7 +1639,7 @@ int autan_wall_distance(const double* triangles, const int64_t* tri_offsets, con
         k_wall_nodes<<<grid, 128>>>(tri, tree + k0, level, node);
         check(cudaGetLastError(), "wall nodes");
       }
-    k_wall_distance<<<blocks(n_points, 128), 128>>>(tri, tree, node, off, n_cases, pts, n_points, out);
+    k_wall_distance<<<blocks(n_points, 128), 128>>>(tri, run_tree, node, off, n_runs, pts, n_points, out);
     check(cudaGetLastError(), "wall distance");
     if (staged)
       check(autan_b200::HostStage::of_device(1)->to_host(distance, out, static_cast<size_t>(n_points) * 8, nullptr,

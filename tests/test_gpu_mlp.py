@@ -121,6 +121,34 @@ def test_wall_distance_through_the_tree(n_tri):
         assert np.array_equal(got[c], np.array(want))
 
 
+def test_wall_distance_of_overlapping_point_ranges():
+    """Point offsets that step back: a point in several cases' ranges is the last one's, as when each
+    case marked its points in turn."""
+    from autan_b200 import _native as N
+    from autan_b200.warmstart import _bind
+
+    rng = np.random.default_rng(3)
+    tris = [rng.normal(size=(n, 9)) + 4.0 * k for k, n in enumerate((40, 7, 90, 3))]
+    toff = np.cumsum([0] + [len(t) for t in tris]).astype(np.int64)
+    poff = np.array([0, 30, 12, 40, 40], dtype=np.int64)  # cases: 0-29, none, 12-39, none
+    n = 40
+    owner = np.zeros(n, dtype=int)
+    for k in range(4):
+        owner[poff[k] : poff[k + 1]] = k
+    pts = np.ascontiguousarray(rng.normal(scale=3.0, size=(3, n)))
+    tri = np.ascontiguousarray(np.concatenate(tris))
+    d = np.zeros(n)
+    err = N.errbuf()
+    import ctypes as C
+
+    N.check(_bind().autan_wall_distance(N.ptr(tri, C.c_double), N.ptr(toff, C.c_int64), N.ptr(pts, C.c_double),
+                                        N.ptr(poff, C.c_int64), 4, n, N.ptr(d, C.c_double), err, len(err)), err)  # fmt: skip
+    assert set(owner) == {0, 2}
+    for i in range(n):
+        (want,) = wall_distance([tris[owner[i]]], [pts[:, i : i + 1]])
+        assert d[i] == want[0], i
+
+
 @pytest.mark.parametrize("rows", [5000, 40000])
 def test_engines_agree(rows):
     """tcgen05 per layer, fused tcgen05 (tensor memory accumulators) and mma.sync: the same BF16

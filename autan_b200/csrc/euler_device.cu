@@ -2872,14 +2872,19 @@ class Impl final : public Stepper {
     d_.wide_ok = (sizeof(C) == 4 && weights_in_range) ? 1 : 0;
     wide_ok_mesh_ = d_.wide_ok;
     d_.stall_polls = 0;
-    check(cudaMallocHost(reinterpret_cast<void**>(&head_), kControlHead), "cudaMallocHost");
-    check(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking), "stream");
-    check(cudaEventCreateWithFlags(&forked_, cudaEventDisableTiming), "event");
-    check(cudaEventCreateWithFlags(&joined_, cudaEventDisableTiming), "event");
-    choose_defaults();
-    ready_plans();
-    trim_plans();
-    check(cudaStreamSynchronize(stream), "create");
+    try {
+      check(cudaMallocHost(reinterpret_cast<void**>(&head_), kControlHead), "cudaMallocHost");
+      check(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking), "stream");
+      check(cudaEventCreateWithFlags(&forked_, cudaEventDisableTiming), "event");
+      check(cudaEventCreateWithFlags(&joined_, cudaEventDisableTiming), "event");
+      choose_defaults();
+      ready_plans();
+      trim_plans();
+      check(cudaStreamSynchronize(stream), "create");
+    } catch (...) {  // (no destructor runs for a constructor that throws)
+      release();
+      throw;
+    }
   }
 
   ~Impl() override {
@@ -2902,9 +2907,8 @@ class Impl final : public Stepper {
       t += static_cast<long long>(b->bytes());
     for (const auto& b : prim_) t += static_cast<long long>(b.bytes());
     t += static_cast<long long>(recon_.bytes());
-    for (const auto& p : grad_plans_)
-      t += static_cast<long long>(p.off.bytes() + p.list.bytes() + p.active.bytes() + p.st.bytes() + p.inc.bytes());
-    for (const auto& p : face_plans_) t += p.bytes();
+    for (const auto& p : grad_plans_) t += static_cast<long long>(p.mem.bytes() + p.active.bytes());
+    for (const auto& p : face_plans_) t += static_cast<long long>(p.mem.bytes() + p.active.bytes());
     return t;
   }
 
@@ -3338,25 +3342,41 @@ class Impl final : public Stepper {
 
   struct GradPlan {
     bool built = false, fits = false;
-    Buffer off, list, st, inc, active;
+    Buffer mem, active;  // one allocation: off, list, st, inc
+    int *off = nullptr, *list = nullptr;
+    C *st = nullptr, *inc = nullptr;
     GradShape shape{};
     int n_active = -1;   // re-packed launches: blocks to launch over (-1: all)
   };
 
   struct FacePlan {
     bool built = false, fits = false;
-    Buffer first, bfirst, rec, face, bface, inc, inc_start, wfirst, walls, active;
-    int faces = 0;          // the most faces of a block
+    Buffer mem, active;  // one allocation: everything below
+    typename P::V* rec = nullptr;
+    uint2* inc = nullptr;
+    int *face = nullptr, *bface = nullptr;
+    const int *first = nullptr, *bfirst = nullptr, *inc_start = nullptr, *wfirst = nullptr, *walls = nullptr;
+    int faces = 0;           // the most faces of a block
     long long interior = 0;  // interior faces over all blocks
-    bool walls_ok = false;  // every boundary face's owner is an owned cell
+    bool walls_ok = false;   // every boundary face's owner is an owned cell
     int n_active = -1;
-    long long bytes() const {
-      long long t = 0;
-      for (const Buffer* b : {&first, &bfirst, &rec, &face, &bface, &inc, &inc_start, &wfirst, &walls, &active})
-        t += static_cast<long long>(b->bytes());
-      return t;
+  };
+
+  // Offsets of arrays in one allocation, each on a 256-byte boundary.
+  struct Carver {
+    size_t total = 0;
+    size_t take(size_t bytes) {
+      const size_t at = total;
+      total += (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
+      return at;
     }
   };
+  template <class T>
+  static T* at_offset(const Buffer& b, size_t at) {
+    return reinterpret_cast<T*>(b.template as<unsigned char>() + at);
+  }
+  // Room for two counts per block of cells: the stage state's memory, which holds nothing between calls.
+  int* block_counts() const { return stage_.as<int>(); }
 
   // A plan, built by `build` (whether its blocks fit) unless it is; null where they do not fit, for want
   // of device memory too: the other forms need none of it.
@@ -3399,13 +3419,13 @@ class Impl final : public Stepper {
     int cap = 1;
     while (cap < most && cap < (1 << 20)) cap <<= 1;
     if (cap > kSortCap) return false;
-    Buffer counts(static_cast<size_t>(nblk) * sizeof(int));
+    int* const counts = block_counts();
     const size_t sm = 2ULL * cap * sizeof(int);
-    launch_smem(kControl, k_grad_blocks<P, false>, nblk, nb, sm, d_, cap, counts.as<int>(),
+    launch_smem(kControl, k_grad_blocks<P, false>, nblk, kSortThreads, sm, d_, nb, cap, counts,
                 static_cast<const int*>(nullptr), static_cast<int*>(nullptr), static_cast<C*>(nullptr),
                 static_cast<C*>(nullptr));
     std::vector<int> n(nblk), off(nblk + 1, 0);
-    check(cudaMemcpyAsync(n.data(), counts.ptr(), counts.bytes(), cudaMemcpyDeviceToHost, stream), "blocks");
+    check(cudaMemcpyAsync(n.data(), counts, n.size() * sizeof(int), cudaMemcpyDeviceToHost, stream), "blocks");
     check(cudaStreamSynchronize(stream), "blocks");
     long long run = 0;
     int largest = 0;
@@ -3425,13 +3445,17 @@ class Impl final : public Stepper {
     }
     for (int c = 0; c < n_; ++c) shape.faces = std::max(shape.faces, inc_.len[c]);
     if (grad_split_bytes<C>(shape, nb) > kBlockSmem) return false;
-    p.off = upload(off, stream);
-    p.list.alloc(std::max<size_t>(1, static_cast<size_t>(run)) * sizeof(int));
-    p.st.alloc(st_e_.bytes());
-    p.inc.alloc(inc_rec_.bytes());
-    launch_smem(kControl, k_grad_blocks<P, true>, nblk, nb, sm, d_, cap, static_cast<int*>(nullptr),
-                static_cast<const int*>(p.off.template as<int>()), p.list.template as<int>(),
-                p.st.template as<C>(), p.inc.template as<C>());
+    Carver cut;
+    const size_t o_st = cut.take(st_e_.bytes()), o_inc = cut.take(inc_rec_.bytes()),
+                 o_off = cut.take(off.size() * sizeof(int)), o_list = cut.take(static_cast<size_t>(run) * sizeof(int));
+    p.mem.alloc(cut.total);
+    p.st = at_offset<C>(p.mem, o_st);
+    p.inc = at_offset<C>(p.mem, o_inc);
+    p.off = at_offset<int>(p.mem, o_off);
+    p.list = at_offset<int>(p.mem, o_list);
+    check(cudaMemcpyAsync(p.off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, stream), "blocks");
+    launch_smem(kControl, k_grad_blocks<P, true>, nblk, kSortThreads, sm, d_, nb, cap, static_cast<int*>(nullptr),
+                static_cast<const int*>(p.off), p.list, p.st, p.inc);
     check(cudaStreamSynchronize(stream), "blocks");
     p.shape = shape;
     return true;
@@ -3485,14 +3509,14 @@ class Impl final : public Stepper {
     int cap = 1;
     while (cap < most && cap < (1 << 20)) cap <<= 1;
     if (cap > kSortCap) return false;
-    Buffer counts(2ULL * nblk * sizeof(int));
+    int* const counts = block_counts();
     const size_t sm = 2ULL * cap * sizeof(int);
-    launch_smem(kControl, k_face_blocks<P, false>, nblk, nb, sm, d_, cap, counts.as<int>(),
+    launch_smem(kControl, k_face_blocks<P, false>, nblk, kSortThreads, sm, d_, nb, cap, counts,
                 static_cast<const int*>(nullptr), static_cast<const int*>(nullptr),
                 static_cast<typename P::V*>(nullptr), static_cast<int*>(nullptr), static_cast<int*>(nullptr),
                 static_cast<uint2*>(nullptr), static_cast<const int*>(nullptr));
     std::vector<int> n(2ULL * nblk), first(nblk + 1, 0), bfirst(nblk + 1, 0);
-    check(cudaMemcpyAsync(n.data(), counts.ptr(), counts.bytes(), cudaMemcpyDeviceToHost, stream), "blocks");
+    check(cudaMemcpyAsync(n.data(), counts, n.size() * sizeof(int), cudaMemcpyDeviceToHost, stream), "blocks");
     check(cudaStreamSynchronize(stream), "blocks");
     long long run = 0, brun = 0;
     for (int b = 0; b < nblk; ++b) {
@@ -3513,18 +3537,6 @@ class Impl final : public Stepper {
       rows += ((inc_.start[s + 1] - inc_.start[s]) / kSlice + 3) / 4 * kSlice;
     }
     start.back() = static_cast<int>(rows);
-    p.first = upload(first, stream);
-    p.bfirst = upload(bfirst, stream);
-    p.inc_start = upload(start, stream);
-    p.rec.alloc(std::max<size_t>(1, static_cast<size_t>(run)) * kFace * sizeof(C));
-    p.face.alloc(std::max<size_t>(1, static_cast<size_t>(run)) * sizeof(int));
-    p.bface.alloc(std::max<size_t>(1, static_cast<size_t>(brun)) * sizeof(int));
-    p.inc.alloc(std::max<size_t>(1, static_cast<size_t>(rows)) * sizeof(uint2));
-    launch_smem(kControl, k_face_blocks<P, true>, nblk, nb, sm, d_, cap, static_cast<int*>(nullptr),
-                static_cast<const int*>(p.first.template as<int>()),
-                static_cast<const int*>(p.bfirst.template as<int>()), p.rec.template as<typename P::V>(),
-                p.face.template as<int>(), p.bface.template as<int>(), p.inc.template as<uint2>(),
-                static_cast<const int*>(p.inc_start.template as<int>()));
     // the boundary faces by their owner's block
     p.walls_ok = true;
     std::vector<int> wfirst(nblk + 1, 0), walls(static_cast<size_t>(std::max(nb_, 1)), 0);
@@ -3549,8 +3561,37 @@ class Impl final : public Stepper {
     for (int b = 0; b < nb_; ++b)
       if (owner_of(b) < n_) walls[at[owner_of(b) / nb]++] = b;
     p.interior = run;
-    p.wfirst = upload(wfirst, stream);
-    p.walls = upload(walls, stream);
+    // the index arrays go up as one
+    std::vector<int> index;
+    size_t at_index[5];
+    {
+      int k = 0;
+      for (const std::vector<int>* v : {&first, &bfirst, &start, &wfirst, &walls}) {
+        at_index[k++] = index.size();
+        index.insert(index.end(), v->begin(), v->end());
+      }
+    }
+    Carver cut;
+    const size_t o_rec = cut.take(static_cast<size_t>(run) * kFace * sizeof(C)),
+                 o_inc = cut.take(static_cast<size_t>(rows) * sizeof(uint2)),
+                 o_face = cut.take(static_cast<size_t>(run) * sizeof(int)),
+                 o_bface = cut.take(static_cast<size_t>(brun) * sizeof(int)),
+                 o_index = cut.take(index.size() * sizeof(int));
+    p.mem.alloc(cut.total);
+    p.rec = at_offset<typename P::V>(p.mem, o_rec);
+    p.inc = at_offset<uint2>(p.mem, o_inc);
+    p.face = at_offset<int>(p.mem, o_face);
+    p.bface = at_offset<int>(p.mem, o_bface);
+    int* const on_device = at_offset<int>(p.mem, o_index);
+    p.first = on_device + at_index[0];
+    p.bfirst = on_device + at_index[1];
+    p.inc_start = on_device + at_index[2];
+    p.wfirst = on_device + at_index[3];
+    p.walls = on_device + at_index[4];
+    check(cudaMemcpyAsync(on_device, index.data(), index.size() * sizeof(int), cudaMemcpyHostToDevice, stream),
+          "blocks");
+    launch_smem(kControl, k_face_blocks<P, true>, nblk, kSortThreads, sm, d_, nb, cap, static_cast<int*>(nullptr), p.first,
+                p.bfirst, p.rec, p.face, p.bface, p.inc, p.inc_start);
     check(cudaStreamSynchronize(stream), "blocks");
     return true;
   }
@@ -3781,11 +3822,8 @@ class Impl final : public Stepper {
       if (some && p.n_active == 0) return;  // every case has stopped
       // first order: only the next step's spectral radius reads boundary states
       const bool walls = carries_walls() && (second_ || last);
-      FaceBlocks<P> g{p.first.template as<int>(), p.bfirst.template as<int>(),
-                      p.rec.template as<typename P::V>(), p.face.template as<int>(),
-                      p.bface.template as<int>(), p.inc.template as<uint2>(),
-                      p.inc_start.template as<int>(), walls ? p.wfirst.template as<int>() : nullptr,
-                      p.walls.template as<int>(), some ? p.active.template as<int>() : nullptr, bs};
+      FaceBlocks<P> g{p.first, p.bfirst, p.rec, p.face, p.bface, p.inc, p.inc_start,
+                      walls ? p.wfirst : nullptr, p.walls, some ? p.active.template as<int>() : nullptr, bs};
       const int nblk = some ? p.n_active : blocks(n_, bs);
       dispatch_faces([&](auto flux, auto planar, auto second) {
         constexpr int F = decltype(flux)::value;
@@ -4212,8 +4250,7 @@ class Impl final : public Stepper {
           const int cells = std::min(bs, kSplitCells);
           const bool some = repacked() && g.n_active >= 0;
           if (some && g.n_active == 0) return;  // every case has stopped
-          GradBlocks<P> gb{g.off.template as<int>(), g.list.template as<int>(), g.st.template as<C>(),
-                           g.inc.template as<C>(), some ? g.active.template as<int>() : nullptr};
+          GradBlocks<P> gb{g.off, g.list, g.st, g.inc, some ? g.active.template as<int>() : nullptr};
           const int nblk = some ? g.n_active : blocks(n_, cells);
           Chain chain(chained_);
           launch_smem(kGradients, k_gradients_split<P, L, D>, nblk, kSplit * cells,

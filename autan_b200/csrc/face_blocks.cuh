@@ -25,18 +25,19 @@ struct FaceBlocks {
 
 // The faces of block b: interior faces f as f, boundary faces b as n_if + b. FILL false: their numbers
 // (interior, boundary) into counts[2 b], counts[2 b + 1]; else the block's lists, records and places.
+// Threads as k_grad_blocks.
 template <class P, bool FILL>
-__global__ void k_face_blocks(Dev<P> d, int cap, int* counts, const int* first, const int* bfirst,
+__global__ void k_face_blocks(Dev<P> d, int nb, int cap, int* counts, const int* first, const int* bfirst,
                               typename P::V* rec, int* face, int* bface, uint2* inc,
                               const int* inc_start) {
   using C = typename P::C;
   using V = typename P::V;
   extern __shared__ int block_keys[];
-  __shared__ int part[257];
+  __shared__ int part[kSortThreads + 1];
   __shared__ int n_keys, n_inner;
   int* key = block_keys;
   int* uniq = block_keys + cap;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int c = static_cast<int>(threadIdx.x) < nb ? static_cast<int>(blockIdx.x) * nb + static_cast<int>(threadIdx.x) : d.n;
   if (threadIdx.x == 0) n_keys = n_inner = 0;
   __syncthreads();
   const long long base = c < d.n ? d.inc_start[c >> 5] + (c & 31) : 0;

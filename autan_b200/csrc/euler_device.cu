@@ -3188,8 +3188,8 @@ class Impl final : public Stepper {
 
   // The autotuner: each candidate launch configuration steps the device state `trial_steps` times
   // (after one untimed step) with event timing; the gradient choices are picked by the gradient
-  // kernel's time, then the face choices by the time of the face kernels and the norms (which
-  // face mode 2 sums inside its gather); whole steps then decide between these and a new handle's
+  // kernel's time, then the face choices by the time of the face kernels, the norms (which face mode 2
+  // sums inside its gather) and the boundary states (which face mode 3 carries); whole steps then decide between these and a new handle's
   // choices. The state is restored after
   // every trial, so tuning leaves the solution unchanged. Returns the tuned ms per step.
   double autotune(double cfl, double dt, bool local, int rk, int trial_steps) override {
@@ -3215,7 +3215,8 @@ class Impl final : public Stepper {
       restore();
       double total = 0.0;
       for (int k = 0; k < 6; ++k) total += ms[k];
-      const double picked = kind == kFaces ? ms[kFaces] + ms[kNorms] : ms[kind];
+      // (the boundary states' own launches: face mode 3 carries them)
+      const double picked = kind == kFaces ? ms[kFaces] + ms[kNorms] + ms[kBoundary] : ms[kind];
       return (kind < 0 ? total : picked) / trial_steps;
     };
     Tuning best = tuning_;
@@ -3609,31 +3610,45 @@ class Impl final : public Stepper {
   }
 
   // The launch choices of a new handle, by owned cells and precision. Measured step times (us, graph,
-  // one B200; tets HLLC, channels AUSM+-up or Roe):
-  //   gradients, split / a thread per cell (two entries in flight, 64 threads): fp32+acc64 channel
-  //   4 743 cells 47 / 90, 60 100 cells 99 / 114, 134 175 cells 217 / 199, tets 108 000 cells
-  //   122 / 105; fp64 channel 13 730 cells 79 / 99, warped hexahedra 24 000 cells 144 / 124. The split
-  //   form issues 1.8 times the instructions, so it wins while the chip has issue slots to spare.
+  // RK3, one B200; tets HLLC, channels AUSM+-up in Morton order unless said, boxes of hexahedra and warped
+  // hexahedra Roe in their generator's order, hexahedra first order):
+  //   Gradients, split / a thread per cell (two entries in flight, 64 threads), the better faces with
+  //   each: fp32+acc64 channels 6 282 cells 47 / 86, 30 368 cells 68 / 99, 60 962 cells 101 / 115,
+  //   100 360 cells 160 / 158, 253 530 cells 334 / 320; tets 24 336 cells 47 / 59, 60 516 cells 74 / 78,
+  //   108 900 cells 121 / 105; fp64 channels 12 130 cells 74 / 96, 24 456 cells 109 / 111, 39 452 cells
+  //   159 / 133; tets 8 100 cells 51 / 55, 24 336 cells 76 / 72. The split form issues 1.8 times the
+  //   instructions, so it wins while the chip has issue slots to spare.
   //   That thread-per-cell form / the staged one: 278 289-cell channel 353 / 466, 2 073 600 tets
   //   1 410 / 1 430.
-  //   Face blocks / store-gather: hexahedra fp64 8 192 cells 38 / 54, fp32+acc64 channels 4 743 cells
-  //   47 / 66, 31 154 cells 68 / 84, 60 100 cells 99 / 109, batched 571 000 cells 665 / 692,
-  //   1 942 000 cells 1 765 / 1 765; tets 2 073 600 cells 1 472 / 1 410 (faces between blocks are
-  //   computed twice); fp64 tets 38 880 cells 87 / 95, 72 000 cells 166 / 152. Cells and threads a
-  //   block: 256 threads to 32 cells at 8 192 cells (38; 128 threads 43), to 64 at 31 154 (68; 32 to
-  //   128: 70), 128 to 64 at 60 100 (99; 128 to 128: 110), 128 to 128 at 134 175 (199; 128 to 64: 207).
-  static constexpr long long kFaceBlockCells = 148LL * (sizeof(C) == 4 ? 4096 : 384);
+  //   Face blocks / store-gather, the better gradients with each: fp32+acc64 channels 6 282 cells 47 / 53,
+  //   30 368 cells 68 / 74, 60 962 cells 106 / 101, 100 360 cells 159 / 160, 146 036 cells 224 / 211 (with
+  //   a thread per cell 229 / 234), 253 530 cells 327 / 320, 606 204 cells 629 / 632; tets 24 336 cells
+  //   47 / 54, 60 516 cells 74 / 78, 108 900 cells 105 / 109, 248 004 cells 231 / 223, 599 076 cells
+  //   485 / 462; hexahedra 8 192 cells 31 / 41, 60 552 cells 49 / 46. fp64 hexahedra 8 192 cells 37 / 47,
+  //   29 768 cells 49 / 49, 56 448 cells 67 / 61; channels 24 456 cells 109 / 115, 39 452 cells 133 / 153,
+  //   56 240 cells 180 / 195; tets 39 204 cells 89 / 92, 57 600 cells 130 / 119; warped hexahedra 29 768
+  //   cells 118 / 122, 56 448 cells 228 / 202 (faces between blocks are computed twice).
+  //   Threads to cells a block: fp32+acc64 256 to 32 at 6 282 cells (47; 256 to 64 49, 128 to 64 51),
+  //   256 to 64 at 30 368 (68; 256 to 128 71), 256 to 128 at 60 962 (106; 128 to 64 107) and 60 516 tets
+  //   (74; 76), 128 to 128 at 108 900 tets (105; 256 to 128 123). fp64 second order 256 to 64 at 6 282 (66;
+  //   256 to 32 74, 128 to 64 68) and 8 100 tets (51; 67), first order, whose faces are half the work, 256
+  //   to 32 at 64 x 64 x 2 hexahedra (RK4, 46; 256 to 64 52; 32 x 32 x 8 RK3 39; 37); 128 to 64 at 24 456
+  //   (109; 128 to 128 119), 128 to 128 at 39 452 (133; 128 to 64 148).
+  //   Cell orders whose blocks are not compact (lines or layers of cells) compute more faces twice. On
+  //   small meshes, where launches count, face blocks win all the same (tets in Cuthill-McKee order,
+  //   30 276 cells, 1.97 computations a face: 47 / 57); beyond 512 cells an SM up to 1.28 they do (the
+  //   100 360 and 108 900 cells above), from 1.60 not: warped hexahedra, 100 352 cells, 1.60 a face:
+  //   190 / 171; channel in Cuthill-McKee order, 100 360 cells, 1.91 a face: 173 / 170.
+  static constexpr long long kFaceBlockCells = 148LL * (sizeof(C) == 4 ? 1024 : 320);
   void choose_defaults() {
     const bool f32 = sizeof(C) == 4;
     const long long per_sm = (static_cast<long long>(n_) + 147) / 148;  // cells
     int nb = 128, threads = 128;
-    if (per_sm <= 64) nb = 32, threads = 256;
-    else if (f32 && per_sm <= 256) nb = 64, threads = 256;
-    else if (!f32 && per_sm <= 128) nb = 32;
-    else if (f32 && per_sm <= 512) nb = 64;
+    if (per_sm <= 64 && (f32 || !second_)) nb = 32, threads = 256;
+    else if (per_sm <= (f32 ? 256 : 64)) nb = 64, threads = 256;
+    else if (f32 && per_sm <= 512) threads = 256;
+    else if (!f32 && per_sm <= 200) nb = 64;
     const FacePlan* f = n_ <= kFaceBlockCells ? face_plan(nb) : nullptr;
-    // cell orders whose blocks are not compact (lines or layers of cells) share too many faces between
-    // blocks: beyond small meshes, where launches count, no more than 1.4 computations a face
     if (f != nullptr && per_sm > 512 && f->interior > 1.4 * nif_) f = nullptr;
     tuning_.face_block = 64;
     tuning_.gather_block = 128;

@@ -413,6 +413,13 @@ def parse_triple(text: str) -> tuple[int, int, int]:
 NO_REFERENCE = "the reference's set-up library (oracle/_ref) is not built: its sources are not here"
 
 
+def why_no_reference(error: OSError) -> str:
+    """Why the CPU sample could not be set up: the reference's library is not built, or the error."""
+    import ref_setup as R  # (cpu_sample has put tests/ on the path)
+
+    return NO_REFERENCE if not R.available() else f"{type(error).__name__}: {error}"
+
+
 def run_reference(args, rank: int, world: int) -> None:
     if rank != 0:
         return
@@ -420,8 +427,8 @@ def run_reference(args, rank: int, world: int) -> None:
     try:
         rate, sample, cores = cpu_throughput(args.steps, max(1, min(args.warmup, 1)), threads,
                                              args.workload)  # fmt: skip
-    except OSError:
-        print(json.dumps({"impl": "reference", "unavailable": NO_REFERENCE}), flush=True)
+    except OSError as e:
+        print(json.dumps({"impl": "reference", "unavailable": why_no_reference(e)}), flush=True)
         return
     line = {
         "impl": "reference",
@@ -862,8 +869,8 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
                                                      args.workload, min_seconds=10.0)  # fmt: skip
                 line["cpu_baseline"] = {"value": rate, "unit": "cell-iterations/s", "cores": cores,
                                         "kind": "port", "sample": sample}  # fmt: skip
-            except OSError:  # oracle/_ref is built only where the reference's sources are
-                line["cpu_baseline"] = {"unavailable": NO_REFERENCE}
+            except OSError as e:  # oracle/_ref is built only where the reference's sources are
+                line["cpu_baseline"] = {"unavailable": why_no_reference(e)}
         print(json.dumps(line), flush=True)
 
 

@@ -66,3 +66,14 @@ def test_nvml_clock_sampler_survives_failed_reads(monkeypatch):
     with bench.clock_sampler("GPU-0") as clocks:
         pass
     assert clocks.summary()["sm_mhz"] is None and clocks.summary()["samples"] == 0
+
+
+def test_the_reference_arm_names_its_own_error(monkeypatch, tmp_path):
+    """`unavailable` says that the reference's library is not built only where it is not: a missing
+    sample, or a library that does not load, is named as it is."""
+    import ref_setup as R
+
+    monkeypatch.setattr(R, "LIB", tmp_path / "libref_setup.so")
+    assert bench.why_no_reference(OSError("x")) == bench.NO_REFERENCE
+    R.LIB.write_bytes(b"")
+    assert bench.why_no_reference(FileNotFoundError("no sample")) == "FileNotFoundError: no sample"

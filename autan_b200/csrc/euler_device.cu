@@ -3359,7 +3359,6 @@ class Impl final : public Stepper {
     const int *first = nullptr, *bfirst = nullptr, *inc_start = nullptr, *wfirst = nullptr, *walls = nullptr;
     int faces = 0;           // the most faces of a block
     long long interior = 0;  // interior faces over all blocks
-    bool walls_ok = false;   // every boundary face's owner is an owned cell
     int n_active = -1;
   };
 
@@ -3538,8 +3537,7 @@ class Impl final : public Stepper {
       rows += ((inc_.start[s + 1] - inc_.start[s]) / kSlice + 3) / 4 * kSlice;
     }
     start.back() = static_cast<int>(rows);
-    // the boundary faces by their owner's block
-    p.walls_ok = true;
+    // the boundary faces by their owner's block (an external ghost's have none)
     std::vector<int> wfirst(nblk + 1, 0), walls(static_cast<size_t>(std::max(nb_, 1)), 0);
     auto owner_of = [&](int b) {
       const C x = bface_host_[static_cast<long long>(b) * kBface + 13];
@@ -3553,10 +3551,8 @@ class Impl final : public Stepper {
         return static_cast<int>(l);
       }
     };
-    for (int b = 0; b < nb_; ++b) {
-      if (owner_of(b) >= n_) p.walls_ok = false;
-      else ++wfirst[owner_of(b) / nb + 1];
-    }
+    for (int b = 0; b < nb_; ++b)
+      if (owner_of(b) < n_) ++wfirst[owner_of(b) / nb + 1];
     for (int b = 0; b < nblk; ++b) wfirst[b + 1] += wfirst[b];
     std::vector<int> at(wfirst.begin(), wfirst.end() - 1);
     for (int b = 0; b < nb_; ++b)
@@ -3597,11 +3593,9 @@ class Impl final : public Stepper {
     return true;
   }
 
-  // Whether the step's face launches also write the next boundary states.
-  bool carries_walls() {
-    const FacePlan* f = block_faces();
-    return f != nullptr && !ranked() && nb_ > 0 && f->walls_ok;
-  }
+  // Whether the step's face launches also write the next boundary states: where every boundary face's
+  // owner is an owned cell.
+  bool carries_walls() { return block_faces() != nullptr && !ranked() && nb_ > 0 && n_ext_ == 0; }
   // Before steps whose face launches carry the boundary states: those of buffer 0, where they start.
   void ready_walls() {
     if (!carries_walls() || walls_ready_) return;

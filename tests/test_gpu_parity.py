@@ -332,6 +332,62 @@ def test_block_forms_are_bit_identical(build, precision):
             assert bits_equal(a, b), (tuning, graph, between)
 
 
+def star_mesh(n, seed):
+    """A hub cell with a face to every other cell, these in a chain, a slip face on every 50th: the
+    arrays of the mesh contract, with smooth values where a geometry would give them (nothing in the
+    loops asks more of them)."""
+    rng = np.random.default_rng(seed)
+    own = np.concatenate([np.zeros(n - 1), np.arange(1, n - 1), np.arange(0, n, 50)]).astype(np.int32)
+    nei = np.concatenate([np.arange(1, n), np.arange(2, n)]).astype(np.int32)
+    ni, nf = nei.size, own.size
+    cells = np.concatenate([own, nei])
+    faces = np.concatenate([np.arange(nf), np.arange(ni)])
+    order = np.lexsort((faces, cells))
+    cell_faces = faces[order].astype(np.int32)
+    offsets = np.concatenate([[0], np.cumsum(np.bincount(cells, minlength=n))])
+    normal = rng.normal(size=(3, nf))
+    # the stencil of a cell: the cells across its faces, and its boundary faces
+    other = np.concatenate([np.concatenate([nei, -np.arange(ni, nf) - 1]), own[:ni]])
+    stencil = other[order].astype(np.int32)
+    md = dict(n_cells=n, n_owned_cells=n, n_faces=nf, n_interior_faces=ni, n_owned_interior_faces=ni,
+              n_owned_faces=nf, owner=own, neighbour=nei, cell_face_offsets=offsets, cell_faces=cell_faces,
+              ghost_owner=np.zeros(0, np.int32), face_normal=normal / np.linalg.norm(normal, axis=0),
+              face_area_magnitude=rng.uniform(0.5, 1.0, nf) / n, face_centroid=rng.uniform(0, 1, (3, nf)),
+              face_moment=np.zeros(0), cell_centroid=rng.uniform(0, 1, (3, n)),
+              cell_volume=rng.uniform(0.9, 1.1, n), stencil_offsets=offsets, stencil=stencil,
+              stencil_lsq_weight=rng.normal(scale=1e-2, size=(3, stencil.size)))  # fmt: skip
+    return md, np.full(nf - ni, 2, dtype=np.uint8), rng
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32+acc64"])
+@pytest.mark.parametrize("n, second", [(420, True), (5400, True), (11000, False)])
+def test_meshes_whose_blocks_do_not_fit(n, second, precision):
+    """A hub cell's rows (from 400 neighbours) or faces (from 5 200 in FP64, 10 300 in FP32) are more
+    than a block's shared memory holds: a new handle, and one asked for blocks, take the other forms
+    and give the oracle's bits."""
+    import dataclasses
+
+    md, kind, rng = star_mesh(n, seed=n)
+    base = cases.vortex_tets(4, 4, 2, precision=precision).scheme
+    scheme = dataclasses.replace(base, second_order=second, limiter=second)
+    rho = 1.0 + 0.05 * rng.uniform(-1, 1, n)
+    v = 0.1 * rng.uniform(-1, 1, (3, n))
+    u0 = np.stack([rho, *(rho * v), (1.0 / 1.4) / 0.4 + 0.5 * rho * (v * v).sum(axis=0)])
+    data = np.zeros((5, kind.size))
+    o = O.Oracle(md, scheme.as_dict(), kind, data)
+    u = u0.copy()
+    norms = [o.step(u, rk=3, cfl=0.3, local=False)[0] for _ in range(2)]
+    assert np.isfinite(u).all()
+    for tuning in (None, dict(grad_mode=6, grad_block=64, face_mode=3, face_block=128, gather_block=256)):
+        with EulerDevice(md, scheme, kind, data, weights=md["stencil_lsq_weight"]) as dev:
+            if tuning:
+                dev.set_tuning(**tuning)
+            dev.upload(u0)
+            dev.step(cfl=0.3, rk=3, n_steps=2)
+            assert bits_equal(dev.download(), u), tuning
+            assert bits_equal(dev.history(2)[0], np.array(norms)), tuning
+
+
 def test_a_handle_keeps_only_the_plans_its_launches_take():
     """The blocks of cells that tuning tried and left are freed: a tuned handle holds the memory of one
     that was given its choices; changing them gives back what the new ones do not take."""

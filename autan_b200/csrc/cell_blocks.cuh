@@ -1,11 +1,11 @@
 // Blocks of consecutive owned cells with the data their neighbourhood needs laid out per block
 // (included by euler_device.cu, inside its namespace).
 //
-// The gradient loop reads about 20 neighbour records a cell, but the cells of a compact block share
-// them: a block of 128 cells of the hybrid channel in Morton order reads about 450 different records
-// besides its own. The block lists those once (GradBlocks::list) and each thread block copies them
-// into shared memory in one round of independent loads; the stencil entries then name a record by its
-// 16-bit place there. What was a chain of dependent gathers through L1 and L2 (row, then record,
+// The gradient loop reads about 23 neighbour records a cell, but the cells of a compact block share
+// them: a block of 32 cells of the hybrid channel in Morton order reads about 180 different records
+// besides its own (64 cells 270). The block lists those once (GradBlocks::list) and each thread block
+// copies them into shared memory in one round of independent loads; the stencil entries then name a
+// record by its place there. What was a chain of dependent gathers through L1 and L2 (row, then record,
 // chunk after chunk) becomes one gather per block and shared-memory reads.
 //
 // Stencil rows and limiter rows keep the sliced layout of the handle's own (32 cells a slice) with

@@ -3221,7 +3221,7 @@ class Impl final : public Stepper {
     };
     Tuning best = tuning_;
     const TrialScope scope = trial_scope(
-        second_, n_, kFaceBlockCells, [&](bool mine) { return any_rank(mine); },
+        second_, n_, kFaceTrialCells, [&](bool mine) { return any_rank(mine); },
         [&](int block) { return grad_plan(block) != nullptr; },
         [&](int block) { return face_plan(block) != nullptr; });
     if (second_) {
@@ -3634,6 +3634,8 @@ class Impl final : public Stepper {
   //   100 360 and 108 900 cells above), from 1.60 not: warped hexahedra, 100 352 cells, 1.60 a face:
   //   190 / 171; channel in Cuthill-McKee order, 100 360 cells, 1.91 a face: 173 / 170.
   static constexpr long long kFaceBlockCells = 148LL * (sizeof(C) == 4 ? 1024 : 320);
+  // ... and to the autotuner, which may still find them by a per cent (606 204-cell Roe channel 619 / 623).
+  static constexpr long long kFaceTrialCells = 148LL * (sizeof(C) == 4 ? 4096 : 384);
   void choose_defaults() {
     const bool f32 = sizeof(C) == 4;
     const long long per_sm = (static_cast<long long>(n_) + 147) / 148;  // cells

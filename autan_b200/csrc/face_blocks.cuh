@@ -88,12 +88,15 @@ __global__ void k_face_blocks(Dev<P> d, int nb, int cap, int* counts, const int*
 // states of its boundary faces: the work of k_face_flux, k_bface_flux, k_gather and the next stage's
 // k_boundary_states in one launch, with the same operations in the same order. Faces between two
 // blocks are computed in both; no flux goes through global memory. blockDim.x is the block's cells
-// or, where the cells alone do not fill the chip, a multiple: its faces then take fewer rounds. Dynamic shared memory: 5 words per
-// face of the largest block (and per cell). On small meshes it is bound by one round of dependent loads
-// and the flux arithmetic of a face or two a thread: the 31 154-cell channel's stage takes 15 us where
-// the four launches took 35. On large ones it issues 15 to 18 % more flux work than it saves in traffic
-// (choose_defaults has the line). Registers bounded for four blocks of 256 per SM: 769 us a step's faces
-// on the 1 942 000-cell channel, for three 858, for five 880.
+// or, where the cells alone do not fill the chip, a multiple: its faces then take fewer rounds. Dynamic
+// shared memory: 5 words per face of the largest block (and per cell). On small meshes it is bound by one
+// round of dependent loads and the flux arithmetic of a face or two a thread: the 31 154-cell channel's
+// stage takes 15 us where the four launches took 35. On large ones it computes a quarter of the interior
+// faces twice (1.27 computations a face at 128 cells a block in Morton order), which costs more than the
+// fluxes' way through memory (choose_defaults has the line); 230 880 cells: 43 us, stalled on the loads of
+// the cells' records (39 % of the warps resident), against 41 for flux and gather. Registers bounded for
+// four blocks of 256 per SM: 769 us a step's faces on the 1 942 000-cell channel, for three 858, for
+// five 880.
 template <class P, bool PLANAR, bool SECOND>
 constexpr int kFaceBlockMin = sizeof(typename P::C) == 4 ? ((PLANAR || !SECOND) ? 4 : 3) : (SECOND ? 1 : 2);
 template <class P, int FLUX, bool PLANAR, bool SECOND>

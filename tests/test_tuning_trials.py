@@ -34,7 +34,7 @@ void run(int r, Rank& me, bool second) {
     met.wait(lock, [&] { return flags[1 - r].size() > k || ended > 0; });
     return mine || (flags[1 - r].size() > k && flags[1 - r][k]);
   };
-  me.scope = trial_scope(second, me.cells, 151552, any, [&](int b) { return (me.fits >> (b / 64)) & 1; },
+  me.scope = trial_scope(second, me.cells, 606208, any, [&](int b) { return (me.fits >> (b / 64)) & 1; },
                          [&](int b) { return (me.fits >> (2 + b / 64)) & 1; });
   std::lock_guard<std::mutex> lock(guard);
   ++ended;
@@ -73,7 +73,7 @@ def trials(tmp_path_factory):
     return run
 
 
-SIZES = [5_000, 75_776, 75_777, 151_552, 151_553, 303_104, 303_105, 2_000_000]
+SIZES = [5_000, 75_776, 75_777, 303_104, 303_105, 606_208, 606_209, 2_000_000]
 
 
 @pytest.mark.parametrize("a, b", list(itertools.combinations_with_replacement(SIZES, 2)))
@@ -100,7 +100,7 @@ def test_a_mesh_alone_tries_what_fits(trials):
     assert not any(g[0] == 6 for g in grads) and not any(f[0] == 3 for f in faces)
     grads, faces = modes(100_000, 31)
     assert any(g[0] == 6 for g in grads) and {f[1] for f in faces if f[0] == 3} == {128}
-    grads, faces = modes(200_000, 31)
-    assert any(g[0] == 6 for g in grads) and not any(f[0] == 3 for f in faces)
+    grads, faces = modes(500_000, 31)
+    assert not any(g[0] == 6 for g in grads) and {f[1] for f in faces if f[0] == 3} == {128}
     grads, faces = modes(2_000_000, 31)
     assert not any(g[0] == 6 for g in grads) and not any(f[0] == 3 for f in faces)

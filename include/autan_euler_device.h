@@ -188,8 +188,8 @@ int autan_euler_device_kernel_times(void* handle, double cfl, double dt, int32_t
  * the warp, [0] (2 or 3) gathers in flight, [7] as for 4, 128 threads per block; 6: five threads per
  * cell, the rows and neighbour records of each block of [1], at most 64, cells in shared memory). A
  * new handle takes face mode 3 and gradient staging 6 on small meshes; a mesh whose blocks do not fit
- * (65 535 or more records or 32 768 faces in one, or its shared memory) takes face mode 1 and staging
- * 0 in their place.
+ * (more than 16 384 entries and incidences of one block's cells, or the launch's shared memory), or
+ * for whose lists there is no device memory, takes face mode 1 and staging 0 in their place.
  * Every choice gives the same bits. No counterpart in the reference beyond its Strategy enum
  * (codegen/include/autan/kernels/strategy.hpp:14-21). */
 int autan_euler_device_set_tuning(void* handle, const int32_t* params, int32_t count, char* err,

@@ -3456,7 +3456,6 @@ class Impl final : public Stepper {
     check(cudaMemcpyAsync(p.off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, stream), "blocks");
     launch_smem(kControl, k_grad_blocks<P, true>, nblk, kSortThreads, sm, d_, nb, cap, static_cast<int*>(nullptr),
                 static_cast<const int*>(p.off), p.list, p.st, p.inc);
-    check(cudaStreamSynchronize(stream), "blocks");
     p.shape = shape;
     return true;
   }
@@ -3589,7 +3588,6 @@ class Impl final : public Stepper {
           "blocks");
     launch_smem(kControl, k_face_blocks<P, true>, nblk, kSortThreads, sm, d_, nb, cap, static_cast<int*>(nullptr), p.first,
                 p.bfirst, p.rec, p.face, p.bface, p.inc, p.inc_start);
-    check(cudaStreamSynchronize(stream), "blocks");
     return true;
   }
 

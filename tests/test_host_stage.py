@@ -56,16 +56,26 @@ int main(int, char** argv) {
   const size_t bytes = std::strtoull(argv[1], nullptr, 10);
   pinned_memory_there = argv[2][0] == '1';
   const bool may_pin = argv[3][0] == '1';
-  std::vector<unsigned char> a(bytes), dev(bytes), b(bytes, 0);
-  for (size_t i = 0; i < bytes; ++i) a[i] = static_cast<unsigned char>(i * 2654435761u >> 13);
+  const int callers = std::atoi(argv[4]);
   auto in = HostStage::of_device(0), out = HostStage::of_device(1);
-  cudaError_t e = in->to_device(dev.data(), a.data(), bytes, nullptr, may_pin);
-  if (e == cudaSuccess) e = out->to_host(b.data(), dev.data(), bytes, nullptr, may_pin);
+  std::atomic<int> errors{0}, wrong{0};
+  auto caller = [&](unsigned seed) {
+    std::vector<unsigned char> a(bytes), dev(bytes), b(bytes, 0);
+    for (size_t i = 0; i < bytes; ++i) a[i] = static_cast<unsigned char>((i + seed) * 2654435761u >> 13);
+    if (in->to_device(dev.data(), a.data(), bytes, nullptr, may_pin) != cudaSuccess) ++errors;
+    if (out->to_host(b.data(), dev.data(), bytes, nullptr, may_pin) != cudaSuccess) ++errors;
+    if (a != b) ++wrong;
+  };
+  std::vector<std::thread> team;
+  for (int c = 1; c < callers; ++c) team.emplace_back(caller, 77u * static_cast<unsigned>(c));
+  caller(0);
+  for (std::thread& t : team) t.join();
+  const int made = copies.load();
   HostRows rows;
   const bool first = rows.get(4096) != nullptr;
   const int asked = pinned_calls;
   const bool again = rows.get(4096) != nullptr;
-  std::printf("%d %d %d %d %d %d\n", e, a == b ? 1 : 0, copies.load(), first ? 1 : 0, again ? 1 : 0,
+  std::printf("%d %d %d %d %d %d\n", errors.load(), wrong.load(), made, first ? 1 : 0, again ? 1 : 0,
               pinned_calls.load() - asked);
 }
 """
@@ -91,8 +101,16 @@ def program(tmp_path_factory):
 @pytest.mark.parametrize("there", [1, 0])
 @pytest.mark.parametrize("may_pin", [1, 0])
 def test_copies_come_back(program, size, there, may_pin):
-    error, same, copies, first, again, asked = program(size, there, may_pin)
-    assert error == 0 and same == 1
+    errors, wrong, copies, first, again, asked = program(size, there, may_pin, 1)
+    assert errors == 0 and wrong == 0
     assert (copies > 2) == bool(there and may_pin and size >= 1 << 20)  # through the slots, or one a way
     # rows of a handle's own: got once, or done without after one refusal
     assert (first, again, asked) == ((1, 1, 0) if there else (0, 0, 0))
+
+
+@pytest.mark.parametrize("size", [(1 << 20) + 12345, (9 << 20) + 7])
+def test_copies_of_several_threads(program, size):
+    """The slots serve one copy at a time and direction; the others go the driver's way."""
+    for _ in range(5):
+        errors, wrong, copies, *_ = program(size, 1, 1, 6)
+        assert errors == 0 and wrong == 0 and copies > 12
